@@ -4,6 +4,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../../include/xplus_b200.h"
 #include "device_common.cuh"
 #include "pcg_kernels.cuh"
@@ -355,6 +357,186 @@ __device__ __forceinline__ void sell_rows_smem(const int2 (&sl)[NS], const int (
                 for (int q = 0; q < CHUNK; ++q) y[k] += v[k][h][q] * (pw[cc[k][h][q] - w0] - pi[k]);
     }
 }
+
+// ---------------------------------------------------------------------------------------
+// The slot stream of one warp through a ring of registers (int16 column offsets).  A warp owns
+// slices sb + warp, sb + warp + wpb, ... and walks them in units: two slices, kUnit slots of each
+// lane's row.  DEPTH units are in flight: as soon as a unit's products are done its registers
+// take the load of the unit DEPTH further on, so the L2 round trip of the slots overlaps the
+// gathers and the row work of the units before it, where loading a group of slices and then
+// gathering from it leaves each phase waiting for the other.  Two slices a unit give the gathers
+// and the chains of products something to overlap with.  The matrix never changes, so the first
+// DEPTH units can be requested before the vectors they meet are final (prime()).
+// What bounds it: the L1/shared-memory pipe (per slice of 8 slots: 12 wavefronts of slot loads,
+// about 21 of gathers with their bank conflicts, 5 of row vectors) and issue slots (about 110
+// instructions a slice).  1108 x 1108 system, us per iteration in A p' + records: groups of four
+// slices loaded, then gathered 9.91; single slices, depth 3 9.08; pairs, depth 2 7.40.
+// ---------------------------------------------------------------------------------------
+template <typename T, int N> struct RawVec;
+template <> struct RawVec<float, 2> { using type = float2; };
+template <> struct RawVec<float, 4> { using type = float4; };
+template <> struct RawVec<unsigned short, 2> { using type = unsigned int; };
+template <> struct RawVec<unsigned short, 4> { using type = uint2; };
+template <typename VT> struct RawOf { using type = unsigned short; };  // BF16, FP16
+template <> struct RawOf<float> { using type = float; };
+
+template <typename VT, int CHUNK, typename R>
+__device__ __forceinline__ float raw_val(const R& r, int q) {
+    if constexpr (std::is_same<VT, float>::value) {
+        if constexpr (CHUNK == 2) return q == 0 ? r.x : r.y;
+        else return q == 0 ? r.x : (q == 1 ? r.y : (q == 2 ? r.z : r.w));
+    } else {
+        uint32_t w;
+        if constexpr (CHUNK == 4) w = q < 2 ? r.x : r.y;
+        else w = r;
+        if constexpr (std::is_same<VT, __half>::value) return (q & 1) ? f16_hi(w) : f16_lo(w);
+        else return (q & 1) ? bf16_hi(w) : bf16_lo(w);
+    }
+}
+// p[off[q]], p a shared-memory byte address, for number q of a chunk's packed int16 offsets: one
+// dot-product instruction makes the address from the packed word
+template <int CHUNK, typename R>
+__device__ __forceinline__ float raw_gather(unsigned p, const R& r, int q) {
+    uint32_t w;
+    if constexpr (CHUNK == 4) w = q < 2 ? r.x : r.y;
+    else w = r;
+    const int at = __dp2a_lo(static_cast<int>(w), (q & 1) ? 0x0400 : 0x0004, static_cast<int>(p));
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+// A register that holds nothing (no instruction): ends the live range of what it held before.
+__device__ __forceinline__ void undefine(float& x) { asm volatile("" : "=f"(x)); }
+__device__ __forceinline__ void undefine(unsigned& x) { asm volatile("" : "=r"(x)); }
+__device__ __forceinline__ void undefine(float2& x) { undefine(x.x); undefine(x.y); }
+__device__ __forceinline__ void undefine(uint2& x) { undefine(x.x); undefine(x.y); }
+__device__ __forceinline__ void undefine(float4& x) { undefine(x.x); undefine(x.y); undefine(x.z); undefine(x.w); }
+
+template <typename VT, int CHUNK, int DEPTH>
+struct SlotRing {
+    using RV = typename RawVec<typename RawOf<VT>::type, CHUNK>::type;
+    using RC = typename RawVec<unsigned short, CHUNK>::type;
+    static constexpr int kUnit = 8;            // slots of a row in one unit
+    static constexpr int HC = kUnit / CHUNK;   // chunks
+    RV v[DEPTH][2][HC];
+    RC c[DEPTH][2][HC];
+    int ls, lc;  // the next unit to request: its first slice and its first slot column
+
+    // The band [sb, se) of the CTA; table: {first slot, width} of its slices.  Slices below sm_end
+    // have their slots in shared memory (mval, mcol: the band's first slot first, table numbers
+    // less m0), the others are at val and col.
+    const VT* val;
+    const short* col;
+    const VT* mval;
+    const short* mcol;
+    const int2* table;
+    int sb, se, sm_end, m0, wpb, lane;
+
+    __device__ __forceinline__ void fetch(int j) {
+        if (ls >= se) return;
+        int wmax = 0;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int s = ls + k * wpb;
+            if (s < se) {
+                const int2 sl = table[s - sb];
+                wmax = max(wmax, sl.y);
+                const bool staged = s < sm_end;  // one (generic) load path for both homes
+                const int off = sl.x - (staged ? m0 : 0) + lc * 32 + lane * CHUNK;
+                const VT* vp = (staged ? mval : val) + off;
+                const short* cp = (staged ? mcol : col) + off;
+#pragma unroll
+                for (int h = 0; h < HC; ++h)
+                    if (lc + h * CHUNK < sl.y) {
+                        v[j][k][h] = *reinterpret_cast<const RV*>(vp + h * 32 * CHUNK);
+                        c[j][k][h] = *reinterpret_cast<const RC*>(cp + h * 32 * CHUNK);
+                    }
+            }
+        }
+        lc += kUnit;
+        if (lc >= wmax) {
+            ls += 2 * wpb;
+            lc = 0;
+        }
+    }
+    __device__ __forceinline__ void prime(int warp) {
+        ls = sb + warp;
+        lc = 0;
+#pragma unroll
+        for (int j = 0; j < DEPTH; ++j) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int h = 0; h < HC; ++h) {
+                    undefine(v[j][k][h]);
+                    undefine(c[j][k][h]);
+                }
+            fetch(j);
+        }
+    }
+    // Products of the primed band with the window pw (row w0 first): row_done(row, p'_row, y) for
+    // each of the warp's rows in slice order, y = sum_j w_ij (p'_j - p'_i) in slot order.
+    template <typename RowDone>
+    __device__ __forceinline__ void run(int warp, const float* pw, int w0, RowDone&& row_done) {
+        int ps = sb + warp, pc = 0;
+        float y0 = 0.0f, y1 = 0.0f;
+        while (ps < se) {
+#pragma unroll
+            for (int j = 0; j < DEPTH; ++j) {
+                if (ps < se) {
+                    const bool second = ps + wpb < se;
+                    const int w_0 = table[ps - sb].y, w_1 = second ? table[ps + wpb - sb].y : 0;
+                    const int row0 = ps * 32 + lane, row1 = second ? row0 + 32 * wpb : row0;
+                    const float* pr0 = pw + (row0 - w0);
+                    const float* pr1 = pw + (row1 - w0);
+                    const unsigned a0 = static_cast<unsigned>(__cvta_generic_to_shared(pr0));
+                    const unsigned a1 = static_cast<unsigned>(__cvta_generic_to_shared(pr1));
+                    const float p0 = *pr0, p1 = *pr1;
+                    if (min(w_0, w_1) - pc > kUnit - CHUNK) {
+                        // both slices fill the unit
+                        float x0[kUnit], x1[kUnit];
+#pragma unroll
+                        for (int q = 0; q < kUnit; ++q) x0[q] = raw_gather<CHUNK>(a0, c[j][0][q / CHUNK], q % CHUNK);
+#pragma unroll
+                        for (int q = 0; q < kUnit; ++q) x1[q] = raw_gather<CHUNK>(a1, c[j][1][q / CHUNK], q % CHUNK);
+#pragma unroll
+                        for (int q = 0; q < kUnit; ++q) {
+                            y0 += raw_val<VT, CHUNK>(v[j][0][q / CHUNK], q % CHUNK) * (x0[q] - p0);
+                            y1 += raw_val<VT, CHUNK>(v[j][1][q / CHUNK], q % CHUNK) * (x1[q] - p1);
+                        }
+                    } else {
+#pragma unroll
+                        for (int h = 0; h < HC; ++h) {
+                            if (pc + h * CHUNK < w_0) {
+                                float x[CHUNK];
+#pragma unroll
+                                for (int q = 0; q < CHUNK; ++q) x[q] = raw_gather<CHUNK>(a0, c[j][0][h], q);
+#pragma unroll
+                                for (int q = 0; q < CHUNK; ++q) y0 += raw_val<VT, CHUNK>(v[j][0][h], q) * (x[q] - p0);
+                            }
+                            if (pc + h * CHUNK < w_1) {
+                                float x[CHUNK];
+#pragma unroll
+                                for (int q = 0; q < CHUNK; ++q) x[q] = raw_gather<CHUNK>(a1, c[j][1][h], q);
+#pragma unroll
+                                for (int q = 0; q < CHUNK; ++q) y1 += raw_val<VT, CHUNK>(v[j][1][h], q) * (x[q] - p1);
+                            }
+                        }
+                    }
+                    fetch(j);
+                    pc += kUnit;
+                    if (pc >= max(w_0, w_1)) {
+                        row_done(row0, p0, y0);
+                        if (second) row_done(row1, p1, y1);
+                        y0 = y1 = 0.0f;
+                        ps += 2 * wpb;
+                        pc = 0;
+                    }
+                }
+            }
+        }
+    }
+};
 
 }  // namespace dev
 }  // namespace xplus

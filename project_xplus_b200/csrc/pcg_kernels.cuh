@@ -42,6 +42,8 @@ struct PcgArgs {
     void* t;                // XT, n_pad: G r temporary
     void* z;                // XT, n_pad: preconditioned residual (GTG mode only)
     double* partial;        // 2 banks x 4 slots x gridDim.x
+    int smem_bytes;         // one-barrier SM-resident kernel: its dynamic shared memory (what the
+                            // vectors leave holds matrix slots)
     unsigned* bar;
     int* err;
     PcgOut* out;
@@ -94,10 +96,12 @@ cudaError_t pcg_launch(const KernelKey& k, const PcgArgs& a, int grid, int tpb, 
 // SM-resident variant (pcg_resident.cu): FP32 vectors in the row-sum form only.
 bool resident_supported(const KernelKey& k);
 int resident_max_slices();
-// Sets the dynamic shared-memory opt-in and reports whether one CTA per SM fits.
+// Sets the dynamic shared-memory opt-in and reports whether one CTA per SM fits, and with how much
+// shared memory to launch: vector_bytes, which it needs, and in the one-barrier kernel up to
+// matrix_bytes more for matrix slots.
 // one_sync: the one-barrier-per-iteration kernel (records {m r, m Ap, p} x 2 generations).
-cudaError_t resident_prepare(const KernelKey& k, int device, size_t smem_bytes, int tpb, bool one_sync,
-                             bool* fits);
+cudaError_t resident_prepare(const KernelKey& k, int device, size_t vector_bytes, size_t matrix_bytes, int tpb,
+                             bool one_sync, bool* fits, size_t* smem_bytes);
 cudaError_t resident_launch(const KernelKey& k, const PcgArgs& a, int grid, int tpb, size_t smem_bytes,
                             bool one_sync, cudaStream_t s, const cudaAccessPolicyWindow& window);
 // GTG-preconditioned persistent kernel (pcg_gtg.cu): FP32 vectors, row-sum form, M^-1 = G^T G

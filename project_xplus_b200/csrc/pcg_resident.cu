@@ -11,11 +11,13 @@
 // breakdown tests and status codes (kernels/cuper_pcg_control_kernel.cpp:1069-1235).
 // pcg_resident1_kernel below needs one grid barrier per iteration instead of two.
 //
-// Shared memory (floats): pw[wn] | r[nb] | ap[nb] | dx[nb] | minv[nb] | rowsum[nb].
+// Shared memory (floats): pw[wn] | r[nb] | ap[nb] | dx[nb] | minv[nb] | rowsum[nb] and, in the
+// one-barrier kernel with int16 offsets, the slots of the band's first slices (values, columns).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "../../include/xplus_b200.h"
@@ -30,6 +32,7 @@ using namespace dev;
 
 constexpr int kResSlices = 1024;  // slice table capacity per CTA
 constexpr int kResNS = 4;         // slices of one warp in flight together in phase A
+constexpr int kRingDepth = 2;     // slot-stream units of one warp in flight (one-barrier kernel)
 
 template <typename VT, int CHUNK, typename IT>
 __global__ void __launch_bounds__(512, 1) pcg_resident_kernel(PcgArgs a) {
@@ -328,15 +331,38 @@ __global__ void __launch_bounds__(512, 1) pcg_resident_kernel(PcgArgs a) {
 // of exchanging z_{k+1} through a second barrier, each row publishes {m r_k, m Ap'_k, p'_k}
 // (double-buffered by generation) and every reader rebuilds p'_{k+1} = (m r_k - alpha m Ap'_k)
 // + beta p'_k for its window with the same fused multiply-adds, bit-identical to the owner's.
+//
+// The slots stream through registers (SlotRing), the first of them requested while the scalars
+// are computed, and what shared memory the vectors leave holds the band's first slices.  us per
+// iteration before -> after that (FP32, 2D): 150^2 4.92 -> 4.20, 301^2 5.59 -> 4.55, 700^2
+// 8.74 -> 7.64, 1108^2 15.3 -> 13.6; BF16 67^3 9.67 -> 9.08.  At 150^2 3.4 us are latency: the
+// block sums (0.4), the grid barrier and totals (2.0), two dependent FP64 divisions.
+// Polling tagged partials instead of a counter barrier and then the totals was slower (5.2
+// against 2.4 us: every CTA then polls 148 x 7 entries).
 // ---------------------------------------------------------------------------------------
 constexpr int kPartials1 = 7;
 
+// The scalar state of one solve, in shared memory: one thread advances it after each reduction and
+// the CTA reads what it needs, so none of it occupies registers through the SpMV.
+struct SolveState {
+    double rz, rr, true_rr, rr_at_replace, tau_true_rr, best, rz_old, pap, alpha, zap;
+    double pend;     // alpha of the update not yet applied to x and r (0: none)
+    float al, be;    // the next iteration's pending alpha and beta as the vectors use them
+    int upd;         // pend != 0
+    int code;        // kGo, kReplace or kStop
+    int status, iterations, replacements, stagnated, mode, stagnant;
+    int drop_replace;
+};
+constexpr int kGo = 0, kReplace = 1, kStop = 2;
+
 template <typename VT, int CHUNK, typename IT>
 __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
-    constexpr int NS = kResNS;
+    // int16 offsets in chunks of 2 or 4 stream through the slot ring; the others load a group of
+    // slices and then gather (ring registers for wider columns would not fit)
+    constexpr bool kRing = std::is_same<IT, short>::value && CHUNK >= 2;
     // halo float4 groups per thread loaded ahead, per record array: as many as fit the
     // 128-register budget without spills (-Xptxas -v)
-    constexpr int kHaloU = std::is_same<VT, float>::value ? 3 : 2;
+    constexpr int kHaloU = !kRing && std::is_same<VT, float>::value ? 3 : 2;
     extern __shared__ float smem[];
     __shared__ double s_red[32 * kPartials1];
     __shared__ double s_tot[kPartials1 + 1];
@@ -344,6 +370,7 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
     __shared__ int2 s_slice[kResSlices];
     __shared__ long long s_clk[6];
     __shared__ int s_exp[2];
+    __shared__ SolveState st;
     GridBarrier bar{a.bar, a.err, a.timeout_ns, 0u, a.debug_skip_block};
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -404,6 +431,38 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
             s_exp[0] = min(lo, r0 + nb);
             s_exp[1] = max(hi, r0);
         }
+    }
+    // the slots of the band's first slices, as many as the launch's shared memory holds beside
+    // the vectors (wn is a multiple of 4 and nb of 32, so both arrays start on 16 bytes)
+    SlotRing<VT, kRing ? CHUNK : 4, kRingDepth> ring;
+    if constexpr (kRing) {
+        const long long m0 = sb < se ? a.slice_ptr[sb] : 0;
+        const long long room = (a.smem_bytes - 4LL * (wn + 5LL * nb)) / static_cast<long long>(sizeof(VT) + sizeof(IT));
+        int lo = 0, hi = max(0, se - sb);  // slices staged
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (a.slice_ptr[sb + mid] - m0 <= room) lo = mid;
+            else hi = mid - 1;
+        }
+        const long long ms = lo > 0 ? a.slice_ptr[sb + lo] - m0 : 0;
+        VT* mval = reinterpret_cast<VT*>(rsv + nb);
+        IT* mcol = reinterpret_cast<IT*>(mval + ms);
+        const uint4* gv = reinterpret_cast<const uint4*>(val + m0);
+        const uint4* gc = reinterpret_cast<const uint4*>(col + m0);
+        const long long nv = ms * static_cast<long long>(sizeof(VT)) / 16, nc = ms * static_cast<long long>(sizeof(IT)) / 16;
+        for (long long i = threadIdx.x; i < nv; i += blockDim.x) reinterpret_cast<uint4*>(mval)[i] = __ldg(gv + i);
+        for (long long i = threadIdx.x; i < nc; i += blockDim.x) reinterpret_cast<uint4*>(mcol)[i] = __ldg(gc + i);
+        ring.val = val;
+        ring.col = col;
+        ring.mval = mval;
+        ring.mcol = mcol;
+        ring.table = s_slice;
+        ring.sb = sb;
+        ring.se = se;
+        ring.sm_end = sb + lo;
+        ring.m0 = static_cast<int>(m0);
+        ring.wpb = wpb;
+        ring.lane = lane;
     }
     if (threadIdx.x == 0) {
         for (int k = 0; k < 5; ++k) s_clk[k] = 0;
@@ -466,13 +525,16 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
     // The halo's records, in float4 groups of the window [w0, w0 + wn) without the own band
     // (w0, r0, nb and wn are multiples of 4): group u < nlo lies below the band, the others
     // above it.  The first kHaloU groups of each thread are loaded into registers as soon as
-    // the grid barrier has made the records final (issue_halo), so the loads overlap the
-    // dot-product totals, the scalar updates and the own band's update.
+    // the reduction has made the records final (issue_halo), so the loads overlap the scalar
+    // updates.
     const int nlo = (r0 - w0) >> 2;
     const int hi0 = (r0 + nb - w0) >> 2;
     const int nh = nlo + (wn >> 2) - hi0;
     const int hbd = static_cast<int>(blockDim.x);
     auto qof = [&](int u) { return u < nlo ? u : hi0 + (u - nlo); };
+    auto prime = [&]() {
+        if constexpr (kRing) ring.prime(warp);
+    };
     float4 hz[kHaloU], hq[kHaloU], hp[kHaloU];
     auto issue_halo = [&](int g) {
         const float4* zr4 = reinterpret_cast<const float4*>(rec_zr(g) + w0);
@@ -481,6 +543,7 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
 #pragma unroll
         for (int v = 0; v < kHaloU; ++v) {
             const int u = threadIdx.x + v * hbd;
+            hz[v] = hq[v] = hp[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (u < nh) {
                 const int qq = qof(u);
                 hz[v] = zr4[qq];
@@ -489,45 +552,187 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
             }
         }
     };
-    bool halo_ready = false;  // hz, hq, hp hold generation gen's halo records
 
-    int gen = 0;
-    residual_phase(true, gen);
+    residual_phase(true, 0);
     if (!bar.sync(&s_flag)) return;
-    issue_halo(gen);
-    halo_ready = true;
+    issue_halo(0);
     grid_totals(cur_bank, 4, s_tot);
-    double rz = s_tot[0], rr = s_tot[1], true_rr = s_tot[2];
-    const double tau_true_rr = a.tau2_rel > 0.0 ? a.tau2_rel * s_tot[3] : a.tau_true_rr;
-    if (lead) a.out->bb = s_tot[3];
-    double rr_at_replace = rr;
-    double pap = 0.0, alpha = 0.0, beta = 0.0;
-    double pend = 0.0;  // alpha of the update not yet applied to x and r (0: none)
-    int status = XPLUS_MAX_ITER, iterations = 0, replacements = 0, stagnated = 0;
-    ReplacePolicy pol(a.restart_on_replace, true_rr);
-    const bool converged_now = true_mode ? (true_rr <= tau_true_rr) : (rr <= a.tau_rr);
     const int flush_every = a.flush_every > 0 ? a.flush_every : 16;
+
+    // breakdown test that opens iteration k (kernels/cuper_pcg_control_kernel.cpp:1069-1235)
+    auto open_iteration = [&](int k) {
+        if (k < a.max_iters && (bad(st.rz) || bad(st.rr) || fabs(st.rz) <= kBreakdownEps)) {
+            st.status = XPLUS_BREAKDOWN;
+            st.code = kStop;
+        } else if (k >= a.max_iters) {
+            st.code = kStop;  // status stays XPLUS_MAX_ITER
+        }
+    };
+    // after the reduction of iteration it: alpha, the next r.z and r.r, and whether to replace
+    auto advance = [&](int it) {
+        st.code = kStop;
+        const double pap = s_tot[0];
+        st.pap = pap;
+        if (bad(pap) || fabs(pap) <= kBreakdownEps) {
+            st.status = XPLUS_BREAKDOWN;
+            return;
+        }
+        st.rz_old = st.rz;
+        const double alpha = st.rz / pap;
+        st.alpha = alpha;
+        if (bad(alpha)) {
+            st.status = XPLUS_BREAKDOWN;
+            return;
+        }
+        st.pend = alpha;
+        const double rz_new = s_tot[1] - 2.0 * alpha * s_tot[2] + alpha * alpha * s_tot[3];
+        const double rr_new = s_tot[4] - 2.0 * alpha * s_tot[5] + alpha * alpha * s_tot[6];
+        st.iterations = it + 1;
+        st.rz = rz_new;
+        st.rr = rr_new;
+        if (bad(rz_new) || bad(rr_new)) {
+            st.status = XPLUS_BREAKDOWN;
+            return;
+        }
+        bool do_replace = false, drop_replace = false;
+        if (true_mode) {
+            if (rr_new <= st.tau_true_rr) do_replace = drop_replace = true;
+            if (a.replace_every > 0 && (it + 1) % a.replace_every == 0) do_replace = true;
+            if (a.replace_drop > 0.0 && rr_new <= a.replace_drop * st.rr_at_replace) do_replace = drop_replace = true;
+        }
+        st.drop_replace = drop_replace;
+        st.zap = 0.0;
+        st.code = do_replace ? kReplace : kGo;
+    };
+    // the residual was replaced: its sums in s_tot
+    auto replaced = [&]() {
+        st.rz = s_tot[0];
+        st.rr = s_tot[1];
+        st.true_rr = s_tot[2];
+        st.pend = 0.0;
+        ++st.replacements;
+        st.rr_at_replace = st.rr;
+        ReplacePolicy pol(a.restart_on_replace, st.best);
+        pol.mode = st.mode;
+        pol.stagnant = st.stagnant;
+        if (pol.after(a.restart_on_replace, st.true_rr, a.stag_factor, a.stag_window)) st.stagnated = 1;
+        st.mode = pol.mode;
+        st.stagnant = pol.stagnant;
+        st.best = pol.best;
+    };
+    // ends iteration it (with `rep`: after a replacement): convergence, beta, the next one's start
+    auto finish = [&](int it, bool rep) {
+        st.code = kStop;
+        if (lead && a.trace && it < a.trace_cap) {
+            double* t = a.trace + 5 * static_cast<size_t>(it);
+            t[0] = st.alpha;
+            t[1] = st.rz / st.rz_old;
+            t[2] = st.rz;
+            t[3] = st.rr;
+            t[4] = sqrt(st.rr > 0.0 ? st.rr : 0.0);
+        }
+        if (true_mode ? (rep && st.true_rr <= st.tau_true_rr) : (st.rr <= a.tau_rr)) {
+            st.status = XPLUS_CONVERGED;
+            return;
+        }
+        if (st.stagnated) return;
+        if (fabs(st.rz_old) <= kBreakdownEps) {
+            st.status = XPLUS_BREAKDOWN;
+            return;
+        }
+        ReplacePolicy pol(a.restart_on_replace, 0.0);
+        pol.mode = st.mode;
+        const double beta = pol.beta(rep, st.drop_replace != 0, st.rz, st.rz_old, st.zap, st.pap);
+        if (bad(beta)) {
+            st.status = XPLUS_BREAKDOWN;
+            return;
+        }
+        st.be = static_cast<float>(beta);
+        st.al = static_cast<float>(st.pend);
+        st.upd = st.pend != 0.0;
+        st.code = kGo;
+        open_iteration(it + 1);
+    };
+
+    if (threadIdx.x == 0) {
+        st.rz = s_tot[0];
+        st.rr = s_tot[1];
+        st.true_rr = s_tot[2];
+        st.tau_true_rr = a.tau2_rel > 0.0 ? a.tau2_rel * s_tot[3] : a.tau_true_rr;
+        if (lead) a.out->bb = s_tot[3];
+        st.rr_at_replace = st.rr;
+        st.pap = st.alpha = st.pend = st.zap = st.rz_old = 0.0;
+        st.al = st.be = 0.0f;
+        st.upd = 0;
+        st.status = XPLUS_MAX_ITER;
+        st.iterations = st.replacements = st.stagnated = st.drop_replace = 0;
+        const ReplacePolicy pol(a.restart_on_replace, st.true_rr);
+        st.mode = pol.mode;
+        st.stagnant = pol.stagnant;
+        st.best = pol.best;
+        st.code = kGo;
+        if (true_mode ? (st.true_rr <= st.tau_true_rr) : (st.rr <= a.tau_rr)) {
+            st.status = XPLUS_CONVERGED;
+            st.code = kStop;
+        } else {
+            open_iteration(0);
+        }
+    }
+    prime();
+    __syncthreads();
     clock(4);
 
-    if (converged_now) {
-        status = XPLUS_CONVERGED;
-    } else {
-        for (int it = 0; it < a.max_iters; ++it) {
-            if (bad(rz) || bad(rr) || fabs(rz) <= kBreakdownEps) {
-                status = XPLUS_BREAKDOWN;
-                break;
-            }
+    if (st.code == kGo) {
+        for (int it = 0;; ++it) {
+            const int gen = it & 1, g1 = gen ^ 1;
             // ---- the previous update and the new p' ----
+            const float al_prev = st.al, be = st.be;
+            const bool upd = st.upd != 0;
+            const bool flush = upd && it % flush_every == 0;
+            // halo [w0, r0) and [r0 + nb, w0 + wn) from the records, in float4 groups: the first
+            // kHaloU groups of each thread were loaded right after the reduction (issue_halo),
+            // a wide halo's others load here
+            auto fill = [&](const float4& z, const float4& q, const float4& p) {
+                float4 o;
+                o.x = __fmaf_rn(be, p.x, __fmaf_rn(-al_prev, q.x, z.x));
+                o.y = __fmaf_rn(be, p.y, __fmaf_rn(-al_prev, q.y, z.y));
+                o.z = __fmaf_rn(be, p.z, __fmaf_rn(-al_prev, q.z, z.z));
+                o.w = __fmaf_rn(be, p.w, __fmaf_rn(-al_prev, q.w, z.w));
+                return o;
+            };
+            {
+                float4* pw4 = reinterpret_cast<float4*>(pw);
+#pragma unroll
+                for (int v = 0; v < kHaloU; ++v) {
+                    const int u = threadIdx.x + v * hbd;
+                    if (u < nh) pw4[qof(u)] = fill(hz[v], hq[v], hp[v]);
+                }
+                const float4* zr4 = reinterpret_cast<const float4*>(rec_zr(gen) + w0);
+                const float4* za4 = reinterpret_cast<const float4*>(rec_za(gen) + w0);
+                const float4* p4 = reinterpret_cast<const float4*>(rec_p(gen) + w0);
+                constexpr int U = kHaloU;
+                int u = threadIdx.x + U * hbd;
+                for (; u + (U - 1) * hbd < nh; u += U * hbd) {
+                    float4 z[U], q[U], p[U];
+#pragma unroll
+                    for (int v = 0; v < U; ++v) {
+                        const int qq = qof(u + v * hbd);
+                        z[v] = zr4[qq];
+                        q[v] = za4[qq];
+                        p[v] = p4[qq];
+                    }
+#pragma unroll
+                    for (int v = 0; v < U; ++v) pw4[qof(u + v * hbd)] = fill(z[v], q[v], p[v]);
+                }
+                for (; u < nh; u += hbd) {
+                    const int qq = qof(u);
+                    pw4[qq] = fill(zr4[qq], za4[qq], p4[qq]);
+                }
+            }
             // Own band, from shared memory: the records this CTA published last iteration are
             // {m r, m Ap', p'} of these very values, so p'_new = fma(beta, p', fma(-alpha, m Ap',
             // m r)) here is bit-identical to what the neighbours rebuild from the records; then
             // the pending update dx += alpha p', r -= alpha Ap'.  Only the halo reads records.
-            if (!halo_ready) issue_halo(gen);
-            halo_ready = false;
-            const float al_prev = static_cast<float>(pend);
-            const bool upd = pend != 0.0;
-            const bool flush = upd && it % flush_every == 0;
-            const float be = static_cast<float>(beta);
             {
                 // four rows per thread and step (float4: pw + r0 - w0, rv, apv, mi and dxv all
                 // start on 16-byte boundaries, w0 being a multiple of 4 and nb of 32); each row's
@@ -572,91 +777,54 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
                     }
                 }
             }
-            pend = 0.0;
-            {
-                // halo [w0, r0) and [r0 + nb, w0 + wn) from the records, in float4 groups:
-                // the first U groups of each thread were loaded right after the grid barrier
-                // (issue_halo), the rest (halos above U * 4 * blockDim.x rows) load here
-                const float4* zr4 = reinterpret_cast<const float4*>(rec_zr(gen) + w0);
-                const float4* za4 = reinterpret_cast<const float4*>(rec_za(gen) + w0);
-                const float4* p4 = reinterpret_cast<const float4*>(rec_p(gen) + w0);
-                float4* pw4 = reinterpret_cast<float4*>(pw);
-                auto fill = [&](const float4& z, const float4& q, const float4& p) {
-                    float4 o;
-                    o.x = __fmaf_rn(be, p.x, __fmaf_rn(-al_prev, q.x, z.x));
-                    o.y = __fmaf_rn(be, p.y, __fmaf_rn(-al_prev, q.y, z.y));
-                    o.z = __fmaf_rn(be, p.z, __fmaf_rn(-al_prev, q.z, z.z));
-                    o.w = __fmaf_rn(be, p.w, __fmaf_rn(-al_prev, q.w, z.w));
-                    return o;
-                };
-#pragma unroll
-                for (int v = 0; v < kHaloU; ++v) {
-                    const int u = threadIdx.x + v * hbd;
-                    if (u < nh) pw4[qof(u)] = fill(hz[v], hq[v], hp[v]);
-                }
-                constexpr int U = kHaloU;
-                const int bd = hbd;
-                int u = threadIdx.x + U * bd;
-                for (; u + (U - 1) * bd < nh; u += U * bd) {
-                    float4 z[U], q[U], p[U];
-#pragma unroll
-                    for (int v = 0; v < U; ++v) {
-                        const int qq = qof(u + v * bd);
-                        z[v] = zr4[qq];
-                        q[v] = za4[qq];
-                        p[v] = p4[qq];
-                    }
-#pragma unroll
-                    for (int v = 0; v < U; ++v) pw4[qof(u + v * bd)] = fill(z[v], q[v], p[v]);
-                }
-                for (; u < nh; u += bd) {
-                    const int qq = qof(u);
-                    pw4[qq] = fill(zr4[qq], za4[qq], p4[qq]);
-                }
-                __syncthreads();
-            }
+            __syncthreads();
             clock(2);
             // ---- Ap' from shared memory, then each row's records of the next generation and
             // its terms of the seven sums (the row's own values only: no CTA barrier between) ----
             {
                 double acc[kPartials1] = {0, 0, 0, 0, 0, 0, 0};
-                const int g1 = gen ^ 1;
                 float* zr1 = rec_zr(g1);
                 float* za1 = rec_za(g1);
                 float* p1 = rec_p(g1);
-                for (int s0 = sb + warp; s0 < se; s0 += NS * wpb) {
-                    int2 sl[NS];
-                    int row[NS];
-                    float pi[NS], y[NS];
-#pragma unroll
-                    for (int k = 0; k < NS; ++k) {
-                        const int s = s0 + k * wpb;
-                        const bool on = s < se;
-                        sl[k] = on ? s_slice[s - sb] : make_int2(0, 0);
-                        row[k] = on ? s * 32 + lane : -1;
-                        pi[k] = on ? pw[row[k] - w0] : 0.0f;
+                auto row_done = [&](int row, float pi, float y) {
+                    const int t = row - r0;
+                    const float ap_ = y * a.val_scale + rsv[t] * pi;
+                    apv[t] = ap_;
+                    const float r_ = rv[t], m = mi[t];
+                    if (row < exp_lo || row >= exp_hi) {
+                        zr1[row] = m * r_;
+                        za1[row] = m * ap_;
+                        p1[row] = pi;
                     }
-                    sell_rows_smem<VT, CHUNK, IT, NS>(sl, row, lane, col, val, pw, w0, pi, y);
+                    const double dr = r_, da = ap_, dm = m;
+                    acc[0] += static_cast<double>(pi) * da;
+                    acc[1] += dm * dr * dr;
+                    acc[2] += dm * dr * da;
+                    acc[3] += dm * da * da;
+                    acc[4] += dr * dr;
+                    acc[5] += dr * da;
+                    acc[6] += da * da;
+                };
+                if constexpr (kRing) {
+                    ring.run(warp, pw, w0, row_done);
+                } else {
+                    constexpr int NS = kResNS;
+                    for (int s0 = sb + warp; s0 < se; s0 += NS * wpb) {
+                        int2 sl[NS];
+                        int row[NS];
+                        float pi[NS], y[NS];
 #pragma unroll
-                    for (int k = 0; k < NS; ++k) {
-                        if (row[k] < 0) continue;
-                        const int t = row[k] - r0;
-                        const float ap_ = y[k] * a.val_scale + rsv[t] * pi[k];
-                        apv[t] = ap_;
-                        const float r_ = rv[t], m = mi[t];
-                        if (row[k] < exp_lo || row[k] >= exp_hi) {
-                            zr1[row[k]] = m * r_;
-                            za1[row[k]] = m * ap_;
-                            p1[row[k]] = pi[k];
+                        for (int k = 0; k < NS; ++k) {
+                            const int s = s0 + k * wpb;
+                            const bool on = s < se;
+                            sl[k] = on ? s_slice[s - sb] : make_int2(0, 0);
+                            row[k] = on ? s * 32 + lane : -1;
+                            pi[k] = on ? pw[row[k] - w0] : 0.0f;
                         }
-                        const double dr = r_, da = ap_, dm = m;
-                        acc[0] += static_cast<double>(pi[k]) * da;
-                        acc[1] += dm * dr * dr;
-                        acc[2] += dm * dr * da;
-                        acc[3] += dm * da * da;
-                        acc[4] += dr * dr;
-                        acc[5] += dr * da;
-                        acc[6] += da * da;
+                        sell_rows_smem<VT, CHUNK, IT, NS>(sl, row, lane, col, val, pw, w0, pi, y);
+#pragma unroll
+                        for (int k = 0; k < NS; ++k)
+                            if (row[k] >= 0) row_done(row[k], pi[k], y[k]);
                     }
                 }
                 clock(3);
@@ -665,103 +833,54 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
             }
             clock(0);
             if (!bar.sync(&s_flag)) return;
-            issue_halo(gen ^ 1);  // the generation just published
-            halo_ready = true;
+            issue_halo(g1);  // the generation just published
             grid_totals(cur_bank, kPartials1, s_tot);
             clock(1);
-            gen ^= 1;
-            pap = s_tot[0];
-            if (bad(pap) || fabs(pap) <= kBreakdownEps) {
-                status = XPLUS_BREAKDOWN;
-                break;
+            if (threadIdx.x == 0) {
+                advance(it);
+                if (st.code == kGo) finish(it, false);
             }
-            const double rz_old = rz;
-            alpha = rz / pap;
-            if (bad(alpha)) {
-                status = XPLUS_BREAKDOWN;
-                break;
-            }
-            pend = alpha;
-            double rz_new = s_tot[1] - 2.0 * alpha * s_tot[2] + alpha * alpha * s_tot[3];
-            double rr_new = s_tot[4] - 2.0 * alpha * s_tot[5] + alpha * alpha * s_tot[6];
-            iterations = it + 1;
-            if (bad(rz_new) || bad(rr_new)) {
-                rz = rz_new;
-                rr = rr_new;
-                status = XPLUS_BREAKDOWN;
-                break;
-            }
-            bool do_replace = false, drop_replace = false;
-            double zap = 0.0;  // z_new . Ap' of a replacement
-            if (true_mode) {
-                if (rr_new <= tau_true_rr) do_replace = drop_replace = true;
-                if (a.replace_every > 0 && iterations % a.replace_every == 0) do_replace = true;
-                if (a.replace_drop > 0.0 && rr_new <= a.replace_drop * rr_at_replace) do_replace = drop_replace = true;
-            }
-            if (do_replace) {
-                halo_ready = false;  // the residual phase rewrites this generation's records
-                apply_update(static_cast<float>(pend));
-                pend = 0.0;
+            prime();  // the next iteration's first slots travel meanwhile
+            __syncthreads();
+            if (st.code == kReplace) {
+                apply_update(static_cast<float>(st.pend));
                 __syncthreads();
                 flush_dx();
                 if (!bar.sync(&s_flag)) return;
-                residual_phase(false, gen);
+                residual_phase(false, g1);
                 if (!bar.sync(&s_flag)) return;
                 grid_totals(cur_bank, 3, s_tot);
                 clock(4);
-                rz_new = s_tot[0];
-                rr_new = s_tot[1];
-                true_rr = s_tot[2];
-                ++replacements;
-                rr_at_replace = rr_new;
-                if (pol.after(a.restart_on_replace, true_rr, a.stag_factor, a.stag_window)) stagnated = 1;
-                if (pol.mode == 4) {
+                if (threadIdx.x == 0) replaced();
+                __syncthreads();
+                if (st.mode == 4) {
                     // z_new . Ap' for the flexible coefficient: a pass of its own, so the
                     // residual phase (and the hot loop around it) stays as in the other modes;
                     // every thread reads back only the records it wrote
                     double acc[1] = {0.0};
                     for (int s = sb + warp; s < se; s += wpb) {
                         const int row = s * 32 + lane;
-                        acc[0] += static_cast<double>(rec_zr(gen)[row]) * static_cast<double>(apv[row - r0]);
+                        acc[0] += static_cast<double>(rec_zr(g1)[row]) * static_cast<double>(apv[row - r0]);
                     }
                     cur_bank = next_bank();
                     publish<1>(acc, s_red, cur_bank);
                     if (!bar.sync(&s_flag)) return;
                     grid_totals(cur_bank, 1, s_tot);
-                    zap = s_tot[0];
+                    if (threadIdx.x == 0) st.zap = s_tot[0];
                 }
+                issue_halo(g1);  // the residual phase rewrote this generation's records
+                if (threadIdx.x == 0) finish(it, true);
+                prime();
+                __syncthreads();
             }
-            if (lead && a.trace && it < a.trace_cap) {
-                double* t = a.trace + 5 * static_cast<size_t>(it);
-                t[0] = alpha;
-                t[1] = rz_new / rz_old;
-                t[2] = rz_new;
-                t[3] = rr_new;
-                t[4] = sqrt(rr_new > 0.0 ? rr_new : 0.0);
-            }
-            rz = rz_new;
-            rr = rr_new;
-            if (true_mode ? (do_replace && true_rr <= tau_true_rr) : (rr <= a.tau_rr)) {
-                status = XPLUS_CONVERGED;
-                break;
-            }
-            if (stagnated) break;
-            if (fabs(rz_old) <= kBreakdownEps) {
-                status = XPLUS_BREAKDOWN;
-                break;
-            }
-            beta = pol.beta(do_replace, drop_replace, rz, rz_old, zap, pap);
-            if (bad(beta)) {
-                status = XPLUS_BREAKDOWN;
-                break;
-            }
+            if (st.code == kStop) break;
         }
     }
-    if (status == XPLUS_MAX_ITER && !true_mode && rr <= a.tau_rr) status = XPLUS_CONVERGED;
+    if (threadIdx.x == 0 && st.status == XPLUS_MAX_ITER && !true_mode && st.rr <= a.tau_rr) st.status = XPLUS_CONVERGED;
 
     // ---- exit: the pending update, dx into x, then the FP64 true residual ----
-    if (pend != 0.0) {
-        apply_update(static_cast<float>(pend));
+    if (st.pend != 0.0) {
+        apply_update(static_cast<float>(st.pend));
         __syncthreads();
     }
     flush_dx();
@@ -784,14 +903,14 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
         grid_totals(cur_bank, 1, s_tot);
         if (threadIdx.x == 0) {
             PcgOut* o = a.out;
-            o->status = status;
-            o->iterations = iterations;
-            o->replacements = replacements;
-            o->stagnated = stagnated;
-            o->rz = rz;
-            o->rr = rr;
-            o->pap = pap;
-            o->alpha = alpha;
+            o->status = st.status;
+            o->iterations = st.iterations;
+            o->replacements = st.replacements;
+            o->stagnated = st.stagnated;
+            o->rz = st.rz;
+            o->rr = st.rr;
+            o->pap = st.pap;
+            o->alpha = st.alpha;
             o->true_rr = s_tot[0];
             o->t_end_ns = globaltimer_ns();
             for (int k = 0; k < 4; ++k) o->t_phase[k] = s_clk[k];
@@ -832,8 +951,8 @@ auto resident_fn(bool one_sync) {
     return one_sync ? pcg_resident1_kernel<VT, CHUNK, IT> : pcg_resident_kernel<VT, CHUNK, IT>;
 }
 
-cudaError_t resident_prepare(const KernelKey& k, int device, size_t smem_bytes, int tpb, bool one_sync,
-                             bool* fits) {
+cudaError_t resident_prepare(const KernelKey& k, int device, size_t vector_bytes, size_t matrix_bytes, int tpb,
+                             bool one_sync, bool* fits, size_t* smem_bytes) {
     *fits = false;
     int optin = 0;
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -846,13 +965,18 @@ cudaError_t resident_prepare(const KernelKey& k, int device, size_t smem_bytes, 
     });
     if (!ok) return cudaSuccess;
     if (e != cudaSuccess) return e;
-    if (smem_bytes + fa.sharedSizeBytes > static_cast<size_t>(optin)) return cudaSuccess;
+    if (vector_bytes + fa.sharedSizeBytes > static_cast<size_t>(optin)) return cudaSuccess;
     if (tpb > fa.maxThreadsPerBlock) return cudaSuccess;
+    // the one-barrier kernel keeps matrix slots in what the vectors leave
+    const size_t limit = static_cast<size_t>(optin) - fa.sharedSizeBytes;
+    const size_t want = one_sync ? std::min(limit, vector_bytes + matrix_bytes) : vector_bytes;
+    // the opt-in belongs to the kernel, not to the handle: always the most a launch may ask for,
+    // so that a handle made later with a smaller need leaves the launches of this one possible
     resident_dispatch(k, [&](auto* vt, auto chunk, auto* it) {
         using VT = std::remove_pointer_t<decltype(vt)>;
         using IT = std::remove_pointer_t<decltype(it)>;
         e = cudaFuncSetAttribute(resident_fn<VT, decltype(chunk)::value, IT>(one_sync),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes));
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit));
     });
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -860,9 +984,10 @@ cudaError_t resident_prepare(const KernelKey& k, int device, size_t smem_bytes, 
         using VT = std::remove_pointer_t<decltype(vt)>;
         using IT = std::remove_pointer_t<decltype(it)>;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, resident_fn<VT, decltype(chunk)::value, IT>(one_sync), tpb, smem_bytes);
+            &per_sm, resident_fn<VT, decltype(chunk)::value, IT>(one_sync), tpb, want);
     });
     if (e != cudaSuccess) return e;
+    *smem_bytes = want;
     *fits = per_sm >= 1;
     return cudaSuccess;
 }

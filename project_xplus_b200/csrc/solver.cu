@@ -54,6 +54,7 @@ struct xplus_pcg {
     double* d_xio = nullptr;
     // control
     double* d_partial = nullptr;
+    unsigned char* d_ctl = nullptr;  // what a solve starts from zeroed: d_bar, d_err, d_out
     unsigned* d_bar = nullptr;
     int* d_err = nullptr;
     xplus::PcgOut* d_out = nullptr;
@@ -91,6 +92,10 @@ struct xplus_pcg {
 namespace xplus {
 
 namespace {
+
+// d_ctl: barrier counter at 0, error flag at 128, PcgOut at 256
+constexpr size_t kCtlBytes = 512;
+static_assert(sizeof(PcgOut) <= kCtlBytes - 256, "PcgOut outgrew its place in the control block");
 
 double round16(double v, int type, double scale) {
     if (type == XPLUS_F16) return static_cast<double>(__half2float(__double2half(v / scale))) * scale;
@@ -581,9 +586,6 @@ void create(const int* row_ptr, const int* col_idx, const double* values, int n,
         h->d_sy = dalloc<unsigned char>(h, np * xs);
         h->d_bio = dalloc<double>(h, static_cast<size_t>(n));
         h->d_xio = dalloc<double>(h, static_cast<size_t>(n));
-        h->d_bar = dalloc<unsigned>(h, 1);
-        h->d_err = dalloc<int>(h, 1);
-        h->d_out = dalloc<PcgOut>(h, 1);
         cudaStream_t st = h->stream;
         const int want_tpb = o.block_threads > 0 ? o.block_threads : 512;
         // SM-resident kernel when its shared-memory band + halo fits one CTA per SM
@@ -598,12 +600,25 @@ void create(const int* row_ptr, const int* col_idx, const double* values, int n,
                     max_nb = std::max(max_nb, (se - sb) * 32);
                 }
                 const size_t smem = sizeof(float) * (static_cast<size_t>(max_wn) + 5 * static_cast<size_t>(max_nb));
+                // the largest band's matrix: slice_ptr at the bands' first slices
+                const int bands = (h->n_slices + per_block - 1) / per_block;
+                std::vector<long long> bp(static_cast<size_t>(bands) + 1);
+                cuda_check(cudaMemcpy2DAsync(bp.data(), sizeof(long long), h->d_slice_ptr,
+                                             static_cast<size_t>(per_block) * sizeof(long long), sizeof(long long),
+                                             static_cast<size_t>(bands), cudaMemcpyDeviceToHost, st), "D2H");
+                cuda_check(cudaStreamSynchronize(st), "sync");
+                bp[static_cast<size_t>(bands)] = h->slots;
+                long long band_slots = 0;
+                for (int b = 0; b < bands; ++b)
+                    band_slots = std::max(band_slots, bp[static_cast<size_t>(b) + 1] - bp[static_cast<size_t>(b)]);
+                const bool stages = h->key.idx16 && o.chunk >= 2;  // the slot ring's layouts
+                const size_t slot_bytes = elem_size(o.value_type) + (h->key.idx16 ? 2 : 4);
                 bool fits = false;
                 h->one_sync = o.barriers_per_iter != 2;
-                cuda_check(resident_prepare(h->key, o.device, smem, want_tpb, h->one_sync, &fits), "resident_prepare");
+                cuda_check(resident_prepare(h->key, o.device, smem, stages ? static_cast<size_t>(band_slots) * slot_bytes : 0, want_tpb,
+                                            h->one_sync, &fits, &h->smem_bytes), "resident_prepare");
                 if (fits) {
                     h->resident = true;
-                    h->smem_bytes = smem;
                     h->grid = res_grid;
                     h->tpb = want_tpb;
                     h->d_win = dalloc<int2>(h, win.size());
@@ -616,6 +631,11 @@ void create(const int* row_ptr, const int* col_idx, const double* values, int n,
             request_l2(h);
         }
         h->d_partial = dalloc<double>(h, static_cast<size_t>(16) * h->grid);
+        // barrier counter, error flag and outcome: one block, zeroed by one memset
+        h->d_ctl = dalloc<unsigned char>(h, kCtlBytes);
+        h->d_bar = reinterpret_cast<unsigned*>(h->d_ctl);
+        h->d_err = reinterpret_cast<int*>(h->d_ctl + 128);
+        h->d_out = reinterpret_cast<PcgOut*>(h->d_ctl + 256);
         h->d_block_clk = dalloc<long long>(h, static_cast<size_t>(4) * h->grid);
         cuda_check(cudaMemsetAsync(h->d_x64, 0, np * sizeof(double), st), "memset");
         cuda_check(cudaStreamSynchronize(st), "sync");
@@ -686,9 +706,8 @@ void enqueue_solve(xplus_pcg* h, double tau, int tau_mode, int max_iters_in, int
         const bool low = h->opts.value_type == XPLUS_BF16 || h->opts.value_type == XPLUS_F16;
         a.restart_on_replace = h->opts.restart_on_replace < 0 ? (low ? 4 : 0) : h->opts.restart_on_replace;
     }
-    cuda_check(cudaMemsetAsync(h->d_bar, 0, sizeof(unsigned), st), "memset");
-    cuda_check(cudaMemsetAsync(h->d_err, 0, sizeof(int), st), "memset");
-    cuda_check(cudaMemsetAsync(h->d_out, 0, sizeof(PcgOut), st), "memset");
+    a.smem_bytes = static_cast<int>(h->smem_bytes);
+    cuda_check(cudaMemsetAsync(h->d_ctl, 0, kCtlBytes, st), "memset");
     cuda_check(cudaEventRecord(h->ev0, st), "event");
     if (h->gtg) {
         a.g_slice_ptr = h->d_g_slice_ptr;
