@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <numeric>
 #include <thread>
 #include <vector>
@@ -166,6 +167,9 @@ struct BackLin {
     const float* dexp;  // optional per-node scalar times wd
     const float* wd;
     int accumulate;
+    const float* mask;  // optional: also masked = dX .* [mask > 0], what the next kernels read
+    float* masked;      // (with keep 0 only this is stored)
+    int keep;
 };
 
 __global__ void __launch_bounds__(256) k_node_backlin(BackLin B, float* __restrict__ dX, int n) {
@@ -206,54 +210,118 @@ __global__ void __launch_bounds__(256) k_node_backlin(BackLin B, float* __restri
                     v.x = fmaf(B.dexp[r], B.wd[c], v.x);
                     v.y = fmaf(B.dexp[r], B.wd[c + 1], v.y);
                 }
-                *out = v;
+                if (B.keep) *out = v;
+                if (B.mask) {
+                    const float2 k = *reinterpret_cast<const float2*>(B.mask + static_cast<size_t>(r) * H + c);
+                    *reinterpret_cast<float2*>(B.masked + static_cast<size_t>(r) * H + c) =
+                        make_float2(k.x > 0.0f ? v.x : 0.0f, k.y > 0.0f ? v.y : 0.0f);
+                }
             }
         }
     }
 }
 
+// The gather kernels below take eight lanes per node, four features (one 16-byte load) each, so a
+// warp keeps four nodes' gathers in flight: with a warp per node, lane = feature, each was a chain
+// of index load and 128-byte gather with nothing beside it (450^2 mesh, n = 202,500: aggregate 69
+// -> 34 us, its backward 79 -> 26 us).  Every feature still adds its neighbours in CSR order.
+constexpr int kNodeLanes = 8;
+
+__device__ __forceinline__ float4 ld_row4(const float* src, int r, int q) {
+    return *reinterpret_cast<const float4*>(src + static_cast<size_t>(r) * H + 4 * q);
+}
+__device__ __forceinline__ void st_row4(float* dst, int r, int q, const float4& v) {
+    *reinterpret_cast<float4*>(dst + static_cast<size_t>(r) * H + 4 * q) = v;
+}
+__device__ __forceinline__ void fma4(float4& acc, float e, const float4& x) {
+    acc.x = fmaf(e, x.x, acc.x);
+    acc.y = fmaf(e, x.y, acc.y);
+    acc.z = fmaf(e, x.z, acc.z);
+    acc.w = fmaf(e, x.w, acc.w);
+}
+
 // s_i = a_i + sum_{j<i} e_ij hl_j + sum_{j>i} e_ij hu_j ;  h_out = h_in + relu(s)
-__global__ void k_aggregate(const int* __restrict__ adj_ptr, const int* __restrict__ adj_col,
+__global__ void __launch_bounds__(256) k_aggregate(const int* __restrict__ adj_ptr, const int* __restrict__ adj_col,
                             const float* __restrict__ adj_e, const float* __restrict__ a,
                             const float* __restrict__ hl, const float* __restrict__ hu,
                             const float* __restrict__ h_in, float* __restrict__ s, float* __restrict__ h_out, int n) {
-    const int lane = threadIdx.x & 31;
-    const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
+    const int q4 = threadIdx.x % kNodeLanes;
+    const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kNodeLanes);
     if (i >= n) return;
-    float acc = a[static_cast<size_t>(i) * H + lane];
-    for (int q = adj_ptr[i]; q < adj_ptr[i + 1]; ++q) {
+    float4 acc = ld_row4(a, i, q4);
+    const float4 hi = ld_row4(h_in, i, q4);
+    const int q1 = adj_ptr[i + 1];
+#pragma unroll 4
+    for (int q = adj_ptr[i]; q < q1; ++q) {
         const int j = adj_col[q];
-        const float* src = j < i ? hl : hu;
-        acc = fmaf(adj_e[q], src[static_cast<size_t>(j) * H + lane], acc);
+        fma4(acc, adj_e[q], ld_row4(j < i ? hl : hu, j, q4));
     }
-    if (s) s[static_cast<size_t>(i) * H + lane] = acc;
-    h_out[static_cast<size_t>(i) * H + lane] = h_in[static_cast<size_t>(i) * H + lane] + fmaxf(acc, 0.0f);
+    if (s) st_row4(s, i, q4, acc);
+    st_row4(h_out, i, q4, make_float4(hi.x + fmaxf(acc.x, 0.0f), hi.y + fmaxf(acc.y, 0.0f), hi.z + fmaxf(acc.z, 0.0f),
+                                      hi.w + fmaxf(acc.w, 0.0f)));
 }
 
-// Edge head and diagonal: warp per row i; lower edges of row i in CSR order.
-__global__ void k_head(const int* __restrict__ low_ptr, const int* __restrict__ low_col,
+// sum_f a_f b_f over the 32 features, lane l of the eight holding f = l + 8 k in k: the pairs of a
+// 32-lane butterfly (f with f ^ 16, then ^ 8, 4, 2, 1) of rounded products
+__device__ __forceinline__ float dot_features(const float (&a)[4], const float (&b)[4]) {
+    const float s0 = __fadd_rn(__fmul_rn(a[0], b[0]), __fmul_rn(a[2], b[2]));
+    const float s1 = __fadd_rn(__fmul_rn(a[1], b[1]), __fmul_rn(a[3], b[3]));
+    float t = s0 + s1;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// Edge head and diagonal: eight lanes per row i (lane l: features l, l + 8, l + 16, l + 24); lower
+// edges of row i in CSR order.
+__global__ void __launch_bounds__(256) k_head(const int* __restrict__ low_ptr, const int* __restrict__ low_col,
                        const float* __restrict__ low_e, const float* __restrict__ low_f, const float* __restrict__ ph,
                        const float* __restrict__ qh,
                        const float* __restrict__ h, const float* __restrict__ isq, const float* __restrict__ wr,
                        ParamOffsets off, float* __restrict__ zpre, float* __restrict__ go, float* __restrict__ gval,
                        float* __restrict__ gd, float* __restrict__ td, float* __restrict__ gdiag, int n) {
-    const int lane = threadIdx.x & 31;
-    const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
-    if (i >= n) return;
-    const float c = wr[off.c + lane], c2 = wr[off.c2 + lane], w = wr[off.w + lane], bw = wr[off.bw];
-    const float phv = ph[static_cast<size_t>(i) * H + lane];
-    for (int k = low_ptr[i]; k < low_ptr[i + 1]; ++k) {
-        const int j = low_col[k];
-        const float zp = phv + qh[static_cast<size_t>(j) * H + lane] + c * low_e[k] + c2 * low_f[k];
-        if (zpre) zpre[static_cast<size_t>(k) * H + lane] = zp;
-        const float g = warp_sum_f(w * fmaxf(zp, 0.0f)) + bw;
-        if (lane == 0) {
+    const int l = threadIdx.x % kNodeLanes;
+    const int at = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kNodeLanes);
+    // the warp's four rows walk together (the sums shuffle): a row beyond the last has no edges
+    const bool there = at < n;
+    const int i = there ? at : n - 1;
+    float c[4], c2[4], w[4], phv[4], hv[4], wd[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int f = l + 8 * k;
+        c[k] = wr[off.c + f];
+        c2[k] = wr[off.c2 + f];
+        w[k] = wr[off.w + f];
+        wd[k] = wr[off.wd + f];
+        phv[k] = ph[static_cast<size_t>(i) * H + f];
+        hv[k] = h[static_cast<size_t>(i) * H + f];
+    }
+    const float bw = wr[off.bw];
+    const int k0 = low_ptr[i], deg = there ? low_ptr[i + 1] - k0 : 0;
+    int steps = deg;
+    steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, 8));
+    steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, 16));
+    for (int e = 0; e < steps; ++e) {
+        const bool on = e < deg;
+        const int k = on ? k0 + e : 0;
+        const int j = on ? low_col[k] : i;
+        float z[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int f = l + 8 * q;
+            const float zp = phv[q] + qh[static_cast<size_t>(j) * H + f] + c[q] * (on ? low_e[k] : 0.0f) +
+                             c2[q] * (on ? low_f[k] : 0.0f);
+            if (zpre && on) zpre[static_cast<size_t>(k) * H + f] = zp;
+            z[q] = fmaxf(zp, 0.0f);
+        }
+        const float g = dot_features(w, z) + bw;
+        if (on && l == 0) {
             go[k] = g;
             gval[k] = g * isq[j];
         }
     }
-    const float t = warp_sum_f(wr[off.wd + lane] * h[static_cast<size_t>(i) * H + lane]) + wr[off.bwd];
-    if (lane == 0) {
+    const float t = dot_features(wd, hv) + wr[off.bwd];
+    if (there && l == 0) {
         const float e = expf(t);
         gd[i] = e;
         td[i] = t;
@@ -329,31 +397,44 @@ __global__ void k_row_sweep(const int* __restrict__ low_ptr, const int* __restri
 //   dexp_i = 2 u_i gd_i / (n B_i) - 2 / n on the diagonal (dL/dt_i).
 // mode 1 (inference): rows of G (gval, gdiag) scaled by 1 / sqrt(B_i), so (G A G^T)_ii = 1.
 // A row with B_i <= 0 or not finite counts in *bad and is left as it is.
-__global__ void k_kaporin(const int* __restrict__ low_ptr, const int* __restrict__ low_col,
+// Eight lanes per row: a row's pattern has a handful of entries, so a warp per row left most lanes
+// idle (450^2 mesh: 126 -> 43 us).  Entry pos belongs to lane pos % 8 and its term to part[pos / 8
+// % 4]: the sum is the 32-lane butterfly's, entry by entry.
+__global__ void __launch_bounds__(256) k_kaporin(const int* __restrict__ low_ptr, const int* __restrict__ low_col,
                           const int* __restrict__ adj_ptr, const int* __restrict__ adj_col,
                           const float* __restrict__ adj_e, const float* __restrict__ go,
                           const float* __restrict__ gd, const float* __restrict__ td, int n, int mode,
                           float* __restrict__ rowloss, float* __restrict__ dgo, float* __restrict__ dexp,
                           float* __restrict__ gval, float* __restrict__ gdiag, int* __restrict__ bad) {
-    const int lane = threadIdx.x & 31;
-    const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
-    if (i >= n) return;
+    const int l = threadIdx.x % kNodeLanes;
+    const int at = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kNodeLanes);
+    const bool there = at < n;
+    const int i = there ? at : n - 1;
     const int lp = low_ptr[i];
     const int m = low_ptr[i + 1] - lp + 1;
-    float part = 0.0f;
-    float u0 = 0.0f;  // u of this lane's first entry (rows of at most 32 entries need no recompute)
-    for (int pos = lane; pos < m; pos += 32) {
-        const float u = kap_u(i, pos, m, lp, low_col, go, gd, adj_ptr, adj_col, adj_e);
-        if (pos == lane) u0 = u;
-        part = fmaf(pos < m - 1 ? go[lp + pos] : gd[i], u, part);
+    float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float u0 = 0.0f;  // u of this lane's first entry (rows of at most 8 entries need no recompute)
+    for (int pos0 = l; pos0 < m; pos0 += 32) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int pos = pos0 + 8 * q;
+            if (pos >= m) break;
+            const float u = kap_u(i, pos, m, lp, low_col, go, gd, adj_ptr, adj_col, adj_e);
+            if (pos == l) u0 = u;
+            part[q] = fmaf(pos < m - 1 ? go[lp + pos] : gd[i], u, part[q]);
+        }
     }
-    const float B = warp_sum_f(part);
+    __syncwarp();
+    float B = (part[0] + part[2]) + (part[1] + part[3]);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) B += __shfl_xor_sync(0xffffffffu, B, o);
+    if (!there) return;
     const bool ok = B > 0.0f && isfinite(B);
     if (!ok) {
-        if (lane == 0) atomicAdd(bad, 1);
+        if (l == 0) atomicAdd(bad, 1);
         if (mode == 0) {
-            for (int pos = lane; pos < m - 1; pos += 32) dgo[lp + pos] = 0.0f;
-            if (lane == 0) {
+            for (int pos = l; pos < m - 1; pos += kNodeLanes) dgo[lp + pos] = 0.0f;
+            if (l == 0) {
                 rowloss[i] = 0.0f;
                 dexp[i] = 0.0f;
             }
@@ -362,18 +443,18 @@ __global__ void k_kaporin(const int* __restrict__ low_ptr, const int* __restrict
     }
     if (mode == 1) {
         const float s = rsqrtf(B);
-        for (int pos = lane; pos < m - 1; pos += 32) gval[lp + pos] *= s;
-        if (lane == 0) gdiag[i] *= s;
+        for (int pos = l; pos < m - 1; pos += kNodeLanes) gval[lp + pos] *= s;
+        if (l == 0) gdiag[i] *= s;
         return;
     }
     const float inv_n = 1.0f / static_cast<float>(n);
     const float c = 2.0f * inv_n / B;
-    for (int pos = lane; pos < m; pos += 32) {
-        const float u = pos == lane ? u0 : kap_u(i, pos, m, lp, low_col, go, gd, adj_ptr, adj_col, adj_e);
+    for (int pos = l; pos < m; pos += kNodeLanes) {
+        const float u = pos == l ? u0 : kap_u(i, pos, m, lp, low_col, go, gd, adj_ptr, adj_col, adj_e);
         if (pos < m - 1) dgo[lp + pos] = c * u;
         else dexp[i] = c * u * gd[i] - 2.0f * inv_n;
     }
-    if (lane == 0) rowloss[i] = logf(B) - 2.0f * td[i];
+    if (l == 0) rowloss[i] = logf(B) - 2.0f * td[i];
 }
 
 // sum partials of v over [count] (FP64 per block, fixed order)
@@ -395,10 +476,14 @@ __global__ void __launch_bounds__(256) k_sum_partial(const float* __restrict__ v
     }
 }
 
-__global__ void k_dsum_final(const double* __restrict__ partial, int blocks, double scale, double* __restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
+__global__ void __launch_bounds__(kRedBlocks) k_dsum_final(const double* __restrict__ partial, int blocks, double scale,
+                                                           double* __restrict__ out) {
+    __shared__ double v[kRedBlocks];
+    if (static_cast<int>(threadIdx.x) < blocks) v[threadIdx.x] = partial[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
         double s = 0.0;
-        for (int b = 0; b < blocks; ++b) s += partial[b];
+        for (int b = 0; b < blocks; ++b) s += v[b];
         *out = s * scale;
     }
 }
@@ -484,165 +569,236 @@ __global__ void k_dG(const int* __restrict__ low_row, const int* __restrict__ lo
     }
 }
 
-// dph_i = sum_{k in low(i)} dgo_k w .* [zpre_k > 0] ; dqh_j = sum_{k in up(j)} (same)
-__global__ void k_head_back(const int* __restrict__ low_ptr, const int* __restrict__ up_ptr, const int* __restrict__ up_k,
-                            const float* __restrict__ zpre, const float* __restrict__ dgo, const float* __restrict__ wr,
-                            ParamOffsets off, float* __restrict__ dph, float* __restrict__ dqh, int n) {
-    const int lane = threadIdx.x & 31;
-    const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
-    if (i >= n) return;
-    const float w = wr[off.w + lane];
-    float a = 0.0f, b = 0.0f;
-    for (int k = low_ptr[i]; k < low_ptr[i + 1]; ++k)
-        if (zpre[static_cast<size_t>(k) * H + lane] > 0.0f) a = fmaf(dgo[k], w, a);
-    for (int q = up_ptr[i]; q < up_ptr[i + 1]; ++q) {
-        const int k = up_k[q];
-        if (zpre[static_cast<size_t>(k) * H + lane] > 0.0f) b = fmaf(dgo[k], w, b);
+constexpr int kEdgeRow = 3 * H + 1;
+
+// dph_i = sum_{k in low(i)} dgo_k w .* [zpre_k > 0] ; dqh_j = sum_{k in up(j)} (same), and in the
+// same pass over the lower edges the edge head's parameter sums, one partial row per block:
+//   dw[f] += dgo relu(zpre_f), dc[f] += dgo w_f [zpre_f > 0] e, dc2[f] += dgo w_f [zpre_f > 0] f,
+//   dbw += dgo;  partial row [dw (H) | dc (H) | dc2 (H) | dbw (1)]
+__global__ void __launch_bounds__(256) k_head_back(const int* __restrict__ low_ptr, const int* __restrict__ up_ptr,
+                            const int* __restrict__ up_k, const float* __restrict__ zpre, const float* __restrict__ dgo,
+                            const float* __restrict__ low_e, const float* __restrict__ low_f,
+                            const float* __restrict__ wr, ParamOffsets off, float* __restrict__ dph,
+                            float* __restrict__ dqh, int n, float* __restrict__ partial) {
+    __shared__ float red[32][kEdgeRow];  // [node slot of the block]
+    const int q4 = threadIdx.x % kNodeLanes, slot = threadIdx.x / kNodeLanes;
+    const float w[4] = {wr[off.w + 4 * q4], wr[off.w + 4 * q4 + 1], wr[off.w + 4 * q4 + 2], wr[off.w + 4 * q4 + 3]};
+    float aw[4] = {}, ac[4] = {}, ac2[4] = {}, ab = 0.0f;
+    for (int i = blockIdx.x * 32 + slot; i < n; i += gridDim.x * 32) {
+        float a[4] = {}, b[4] = {};
+        const int k1 = low_ptr[i + 1];
+#pragma unroll 2
+        for (int k = low_ptr[i]; k < k1; ++k) {
+            const float4 z4 = ld_row4(zpre, k, q4);
+            const float z[4] = {z4.x, z4.y, z4.z, z4.w};
+            const float d = dgo[k], e = low_e[k], f = low_f[k];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                aw[v] = fmaf(d, fmaxf(z[v], 0.0f), aw[v]);
+                if (z[v] > 0.0f) {
+                    a[v] = fmaf(d, w[v], a[v]);
+                    ac[v] = fmaf(d * w[v], e, ac[v]);
+                    ac2[v] = fmaf(d * w[v], f, ac2[v]);
+                }
+            }
+            ab += d;
+        }
+        const int u1 = up_ptr[i + 1];
+#pragma unroll 4
+        for (int q = up_ptr[i]; q < u1; ++q) {
+            const int k = up_k[q];
+            const float4 z4 = ld_row4(zpre, k, q4);
+            const float d = dgo[k];
+            if (z4.x > 0.0f) b[0] = fmaf(d, w[0], b[0]);
+            if (z4.y > 0.0f) b[1] = fmaf(d, w[1], b[1]);
+            if (z4.z > 0.0f) b[2] = fmaf(d, w[2], b[2]);
+            if (z4.w > 0.0f) b[3] = fmaf(d, w[3], b[3]);
+        }
+        st_row4(dph, i, q4, make_float4(a[0], a[1], a[2], a[3]));
+        st_row4(dqh, i, q4, make_float4(b[0], b[1], b[2], b[3]));
     }
-    dph[static_cast<size_t>(i) * H + lane] = a;
-    dqh[static_cast<size_t>(i) * H + lane] = b;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        red[slot][4 * q4 + v] = aw[v];
+        red[slot][H + 4 * q4 + v] = ac[v];
+        red[slot][2 * H + 4 * q4 + v] = ac2[v];
+    }
+    if (q4 == 0) red[slot][3 * H] = ab;
+    __syncthreads();
+    for (int o = threadIdx.x; o < kEdgeRow; o += blockDim.x) {
+        float t = 0.0f;
+        for (int q = 0; q < 32; ++q) t += red[q][o];
+        partial[static_cast<size_t>(blockIdx.x) * kEdgeRow + o] = t;
+    }
 }
 
-// Layer backward through the aggregation: ds = dh .* [s > 0] for the own row, and
+// Layer backward through the aggregation, ds = dh .* [s > 0] given:
 // dhl_j = sum_{i in N(j), i > j} e_ij ds_i ; dhu_j = sum_{i in N(j), i < j} e_ij ds_i.
-__global__ void k_agg_back(const int* __restrict__ adj_ptr, const int* __restrict__ adj_col,
-                           const float* __restrict__ adj_e, const float* __restrict__ dh, const float* __restrict__ s,
-                           float* __restrict__ ds, float* __restrict__ dhl, float* __restrict__ dhu, int n) {
-    const int lane = threadIdx.x & 31;
-    const int j = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
+__global__ void __launch_bounds__(256) k_agg_back(const int* __restrict__ adj_ptr, const int* __restrict__ adj_col,
+                           const float* __restrict__ adj_e, const float* __restrict__ ds, float* __restrict__ dhl,
+                           float* __restrict__ dhu, int n) {
+    const int q4 = threadIdx.x % kNodeLanes;
+    const int j = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kNodeLanes);
     if (j >= n) return;
-    const size_t oj = static_cast<size_t>(j) * H + lane;
-    ds[oj] = s[oj] > 0.0f ? dh[oj] : 0.0f;
-    float l = 0.0f, u = 0.0f;
-    for (int q = adj_ptr[j]; q < adj_ptr[j + 1]; ++q) {
+    float4 l = make_float4(0.0f, 0.0f, 0.0f, 0.0f), u = l;
+    const int q1 = adj_ptr[j + 1];
+#pragma unroll 4
+    for (int q = adj_ptr[j]; q < q1; ++q) {
         const int i = adj_col[q];
-        const size_t oi = static_cast<size_t>(i) * H + lane;
-        const float d = s[oi] > 0.0f ? dh[oi] : 0.0f;
-        if (i > j) l = fmaf(adj_e[q], d, l);
-        else u = fmaf(adj_e[q], d, u);
+        const float4 d = ld_row4(ds, i, q4);
+        if (i > j) fma4(l, adj_e[q], d);
+        else fma4(u, adj_e[q], d);
     }
-    dhl[oj] = l;
-    dhu[oj] = u;
-}
-
-// dX_in = dX .* [X > 0]  (relu of the input layer: h0 > 0 iff its pre-activation > 0)
-__global__ void k_relu_mask(const float* __restrict__ d, const float* __restrict__ x, float* __restrict__ out, long long count) {
-    const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t < count) out[t] = x[t] > 0.0f ? d[t] : 0.0f;
+    st_row4(dhl, j, q4, l);
+    st_row4(dhu, j, q4, u);
 }
 
 // ---- deterministic reductions ----
-// partial[b][o*KB + k] = sum_{i in chunk b} D[i][o] X[i][k]; partial[b][32*KB + o] = sum D[i][o]
-template <int KB>
-__global__ void __launch_bounds__(256) k_outer_partial(const float* __restrict__ D, const float* __restrict__ X,
-                                                       int n, int chunk, float* __restrict__ partial) {
-    __shared__ float Ds[32][H + 1];
-    __shared__ float Xs[32][KB + 1];
-    constexpr int NOUT = H * KB + H;
-    constexpr int PER = (NOUT + 255) / 256;
-    float acc[PER];
+// Every weight gradient is a sum over nodes (or edges) of products; each kernel below leaves one
+// partial row per block, and k_grad_final adds all rows of all of them in one launch.
+constexpr int kGradBlocks = 296;     // blocks (partial rows) of each: two per SM
+constexpr int kOuterRow = H * H + H; // dW [H][H] | db [H]
+
+// Partial rows of dW_m = D_m^T X (and db_m = sum_i D_m[i]) for matrix m = blockIdx.y.  Each warp
+// keeps a whole 32 x 32 accumulator in registers (4 x 8 per lane) and walks nodes, four in flight:
+// three loads for 32 FMAs a lane and node, so the FMA pipes bound it, and the 104 MB that a layer
+// reads.  (A 32-node tile in shared memory with one output per thread and step read two
+// shared-memory words per FMA: 150 us per matrix at n = 202,500, now 23.)
+struct OuterArgs {
+    const float* D[3];
+    float* partial[3];
+};
+__global__ void __launch_bounds__(256, 2) k_outer_partial(OuterArgs o, const float* __restrict__ X, int n) {
+    __shared__ float red[8][kOuterRow];
+    const float* __restrict__ D = blockIdx.y == 0 ? o.D[0] : (blockIdx.y == 1 ? o.D[1] : o.D[2]);
+    float* __restrict__ partial = blockIdx.y == 0 ? o.partial[0] : (blockIdx.y == 1 ? o.partial[1] : o.partial[2]);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = lane >> 2, j = lane & 3;  // rows 4 i .. 4 i + 3 of dW, columns 8 j .. 8 j + 7
+    float acc[4][8] = {}, bias[4] = {};
+    const int W = gridDim.x * 8;
+    for (int r0 = blockIdx.x * 8 + warp; r0 < n; r0 += 4 * W) {
+        float4 d[4], x[4][2];
 #pragma unroll
-    for (int q = 0; q < PER; ++q) acc[q] = 0.0f;
-    const int i0 = blockIdx.x * chunk, i1 = min(n, i0 + chunk);
-    for (int base = i0; base < i1; base += 32) {
-        __syncthreads();
-        for (int q = threadIdx.x; q < 32 * H; q += 256) {
-            const int r = q / H, f = q % H, i = base + r;
-            Ds[r][f] = i < i1 ? D[static_cast<size_t>(i) * H + f] : 0.0f;
+        for (int v = 0; v < 4; ++v) {
+            const int r = r0 + v * W;
+            if (r < n) {
+                d[v] = ld_row4(D, r, i);
+                x[v][0] = ld_row4(X, r, 2 * j);
+                x[v][1] = ld_row4(X, r, 2 * j + 1);
+            } else {
+                d[v] = x[v][0] = x[v][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
         }
-        for (int q = threadIdx.x; q < 32 * KB; q += 256) {
-            const int r = q / KB, f = q % KB, i = base + r;
-            Xs[r][f] = i < i1 ? X[static_cast<size_t>(i) * KB + f] : 0.0f;
-        }
-        __syncthreads();
 #pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int o = threadIdx.x + 256 * q;
-            if (o < H * KB) {
-                const int a = o / KB, k = o % KB;
-                float s = acc[q];
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r) s = fmaf(Ds[r][a], Xs[r][k], s);
-                acc[q] = s;
-            } else if (o < NOUT) {
-                const int a = o - H * KB;
-                float s = acc[q];
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r) s += Ds[r][a];
-                acc[q] = s;
+        for (int v = 0; v < 4; ++v) {
+            const float dv[4] = {d[v].x, d[v].y, d[v].z, d[v].w};
+            const float xv[8] = {x[v][0].x, x[v][0].y, x[v][0].z, x[v][0].w, x[v][1].x, x[v][1].y, x[v][1].z, x[v][1].w};
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(dv[p], xv[q], acc[p][q]);
+                bias[p] += dv[p];
             }
         }
     }
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int o = threadIdx.x + 256 * q;
-        if (o < NOUT) partial[static_cast<size_t>(blockIdx.x) * NOUT + o] = acc[q];
+    for (int p = 0; p < 4; ++p) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) red[warp][(4 * i + p) * H + 8 * j + q] = acc[p][q];
+        if (j == 0) red[warp][H * H + 4 * i + p] = bias[p];
     }
-}
-
-// grad[dst_w + o] = sum_b partial[b][o] for o < nw ; grad[dst_b + o] = sum_b partial[b][nw + o] (dst_b >= 0)
-__global__ void k_partial_final(const float* __restrict__ partial, int blocks, int stride, int nw, int nb,
-                                float* __restrict__ grad, int dst_w, int dst_b) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nw + nb) return;
-    float s = 0.0f;
-    for (int b = 0; b < blocks; ++b) s += partial[static_cast<size_t>(b) * stride + o];
-    if (o < nw) grad[dst_w + o] = s;
-    else if (dst_b >= 0) grad[dst_b + (o - nw)] = s;
-}
-
-// Edge-head parameter partials over lower edges (warp per edge, grid-stride):
-//   dw[f] += dgo relu(zpre_f), dc[f] += dgo w_f [zpre_f > 0] e, dc2[f] += dgo w_f [zpre_f > 0] f,
-//   dbw += dgo;  partial row layout [dw (H) | dc (H) | dc2 (H) | dbw (1)]
-constexpr int kEdgeRow = 3 * H + 1;
-__global__ void __launch_bounds__(256) k_edge_partial(const float* __restrict__ zpre, const float* __restrict__ dgo,
-                                                      const float* __restrict__ low_e, const float* __restrict__ low_f,
-                                                      const float* __restrict__ wr, ParamOffsets off, int n_low,
-                                                      float* __restrict__ partial) {
-    __shared__ float red[8][kEdgeRow];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float w = wr[off.w + lane];
-    float aw = 0.0f, ac = 0.0f, ac2 = 0.0f, ab = 0.0f;
-    for (int k = blockIdx.x * 8 + warp; k < n_low; k += gridDim.x * 8) {
-        const float z = zpre[static_cast<size_t>(k) * H + lane];
-        const float d = dgo[k];
-        aw = fmaf(d, fmaxf(z, 0.0f), aw);
-        if (z > 0.0f) {
-            ac = fmaf(d * w, low_e[k], ac);
-            ac2 = fmaf(d * w, low_f[k], ac2);
-        }
-        ab += d;
-    }
-    red[warp][lane] = aw;
-    red[warp][H + lane] = ac;
-    red[warp][2 * H + lane] = ac2;
-    if (lane == 0) red[warp][3 * H] = ab;
     __syncthreads();
-    for (int o = threadIdx.x; o < kEdgeRow; o += blockDim.x) {
+    for (int t = threadIdx.x; t < kOuterRow; t += blockDim.x) {
         float s = 0.0f;
-        for (int q = 0; q < 8; ++q) s += red[q][o];
-        partial[static_cast<size_t>(blockIdx.x) * kEdgeRow + o] = s;
+#pragma unroll
+        for (int v = 0; v < 8; ++v) s += red[v][t];
+        partial[static_cast<size_t>(blockIdx.x) * kOuterRow + t] = s;
     }
 }
 
-// Node partials of a weighted column sum: out[f] = sum_i coef_i X[i][f], out[H] = sum_i coef_i
+// Partial rows of NC coefficient-weighted column sums, sum_i coef_i[c] X[i][f], and of a plain sum:
+// NC = 1 (coef one value a node): [sum coef X (H) | sum coef (1)];  NC = 2 (the input layer, coef the
+// node inputs): [sum X coef[c] as [f][c] (2 H) | sum X (H)].  Lane = feature, four nodes in flight.
+template <int NC>
 __global__ void __launch_bounds__(256) k_vec_partial(const float* __restrict__ coef, const float* __restrict__ X, int n,
                                                      float* __restrict__ partial) {
-    __shared__ float red[8][H + 1];
+    constexpr int ROW = NC == 1 ? H + 1 : 3 * H;
+    __shared__ float red[8][3 * H];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float aw = 0.0f, ab = 0.0f;
-    for (int i = blockIdx.x * 8 + warp; i < n; i += gridDim.x * 8) {
-        const float c = coef[i];
-        aw = fmaf(c, X[static_cast<size_t>(i) * H + lane], aw);
-        ab += c;
+    float s0 = 0.0f, s1 = 0.0f, sb = 0.0f;
+    const int W = gridDim.x * 8;
+    for (int r0 = blockIdx.x * 8 + warp; r0 < n; r0 += 4 * W) {
+        float x[4], c0[4], c1[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const int r = r0 + v * W;
+            const bool on = r < n;
+            x[v] = on ? X[static_cast<size_t>(r) * H + lane] : 0.0f;
+            c0[v] = on ? coef[static_cast<size_t>(r) * NC] : 0.0f;
+            c1[v] = NC == 2 && on ? coef[static_cast<size_t>(r) * NC + 1] : 0.0f;
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            s0 = fmaf(c0[v], x[v], s0);
+            if (NC == 2) s1 = fmaf(c1[v], x[v], s1);
+            sb += NC == 2 ? x[v] : c0[v];
+        }
     }
-    red[warp][lane] = aw;
-    if (lane == 0) red[warp][H] = ab;
+    if (NC == 2) {
+        red[warp][2 * lane] = s0;
+        red[warp][2 * lane + 1] = s1;
+        red[warp][2 * H + lane] = sb;
+    } else {
+        red[warp][lane] = s0;
+        if (lane == 0) red[warp][H] = sb;
+    }
     __syncthreads();
-    for (int o = threadIdx.x; o < H + 1; o += blockDim.x) {
+    for (int o = threadIdx.x; o < ROW; o += blockDim.x) {
         float s = 0.0f;
         for (int q = 0; q < 8; ++q) s += red[q][o];
-        partial[static_cast<size_t>(blockIdx.x) * (H + 1) + o] = s;
+        partial[static_cast<size_t>(blockIdx.x) * ROW + o] = s;
+    }
+}
+
+// grad[dst + o] = sum over the rows b < kGradBlocks of partial[b * stride + o], o < count, for every
+// segment.  32 outputs a block, eight row groups each summed in order, then the groups in order.
+struct GradSegment {
+    const float* partial;
+    int stride, count, dst;
+};
+struct GradTable {
+    GradSegment seg[24];
+    int count = 0;
+    void add(const float* partial, int stride, int count_, int dst) { seg[count++] = {partial, stride, count_, dst}; }
+    int blocks() const {
+        int b = 0;
+        for (int k = 0; k < count; ++k) b += (seg[k].count + 31) / 32;
+        return b;
+    }
+};
+__global__ void __launch_bounds__(256) k_grad_final(GradTable t, float* __restrict__ grad) {
+    __shared__ float red[8][32];
+    int b = blockIdx.x, k = 0;
+    for (; k < t.count - 1; ++k) {
+        const int nb = (t.seg[k].count + 31) / 32;
+        if (b < nb) break;
+        b -= nb;
+    }
+    const GradSegment s = t.seg[k];
+    const int o = b * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
+    float v = 0.0f;
+    if (o < s.count) {
+        constexpr int PER = kGradBlocks / 8;
+#pragma unroll 8
+        for (int r = 0; r < PER; ++r) v += s.partial[static_cast<size_t>(g * PER + r) * s.stride + o];
+    }
+    red[g][threadIdx.x & 31] = v;
+    __syncthreads();
+    if (g == 0 && o < s.count) {
+        float f = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) f += red[q][threadIdx.x];
+        grad[s.dst + o] = f;
     }
 }
 
@@ -1120,6 +1276,11 @@ void DevGraph::upload(const HostGraph& g, Arena& ar, cudaStream_t st) {
     pos_diag = up(ar, g.pos_diag, st);
 }
 
+// the partial rows of all gradient sums, one block's worth: eleven outer products, the edge head,
+// the diagonal head and the input layer
+constexpr int kOuters = 2 + 3 * kLayers;
+constexpr int kPartialRow = kOuters * kOuterRow + kEdgeRow + (H + 1) + 3 * H;
+
 void Work::alloc(Arena& ar, int max_n, int max_low, int K_, bool train) {
     K = K_;
     const size_t nH = static_cast<size_t>(max_n) * H, lH = static_cast<size_t>(max_low) * H;
@@ -1148,13 +1309,13 @@ void Work::alloc(Arena& ar, int max_n, int max_low, int K_, bool train) {
     dgo = ar.get<float>(static_cast<size_t>(max_low));
     dexp = ar.get<float>(static_cast<size_t>(max_n));
     dh = ar.get<float>(nH);
-    dh2 = ar.get<float>(nH);
+    ds2 = ar.get<float>(nH);
     ds = ar.get<float>(nH);
     dhl = ar.get<float>(nH);
     dhu = ar.get<float>(nH);
     dph = ar.get<float>(nH);
     dqh = ar.get<float>(nH);
-    partial = ar.get<float>(static_cast<size_t>(kRedBlocks) * (H * H + H));
+    partial = ar.get<float>(static_cast<size_t>(kGradBlocks) * kPartialRow);
     dpartial = ar.get<double>(static_cast<size_t>(kRedBlocks));
     loss = ar.get<double>(1);
 }
@@ -1174,7 +1335,7 @@ static void kcheck_status(cudaError_t e, const char* what) {
 void forward(const DevGraph& g, const float* wr, Work& w, bool train, cudaStream_t st) {
     const ParamOffsets off = param_offsets();
     const int n = g.n;
-    const int nodes_blocks = blocks_for(static_cast<long long>(n) * 32, 256);
+    const int nodes_blocks = blocks_for(static_cast<long long>(n) * kNodeLanes, 256);
     const int lin_blocks = std::min(blocks_for(n, 8 * 16), 148 * 8);  // 8 warps of 16-node tiles
     k_input<<<blocks_for(static_cast<long long>(n) * H, 256), 256, 0, st>>>(g.x, wr + off.W0, wr + off.b0, w.h[0], n);
     kcheck("gnn input");
@@ -1203,7 +1364,7 @@ void refine_rows(const DevGraph& g, Work& w, int sweeps, cudaStream_t st) {
 }
 
 void normalize_rows(const DevGraph& g, Work& w, cudaStream_t st) {
-    const int nodes_blocks = blocks_for(static_cast<long long>(g.n) * 32, 256);
+    const int nodes_blocks = blocks_for(static_cast<long long>(g.n) * kNodeLanes, 256);
     kcheck_status(cudaMemsetAsync(w.bad, 0, sizeof(int), st), "gnn memset");
     k_kaporin<<<nodes_blocks, 256, 0, st>>>(g.low_ptr, g.low_col, g.adj_ptr, g.adj_col, g.adj_e, w.go, w.gd, w.td,
                                             g.n, 1, nullptr, nullptr, nullptr, w.gval, w.gdiag, w.bad);
@@ -1220,39 +1381,17 @@ void g_to_low(const DevGraph& g, const Work& w, double* d_glow, cudaStream_t st)
     kcheck("gnn g_low");
 }
 
-static void outer_grad(const float* D, const float* X, int kb, int n, Work& w, float* grad, int dst_w, int dst_b,
-                       cudaStream_t st) {
-    const int chunk = std::max(32, ((n + kRedBlocks - 1) / kRedBlocks + 31) / 32 * 32);
-    const int blocks = (n + chunk - 1) / chunk;
-    const int nw = H * kb;
-    if (kb == H) k_outer_partial<H><<<blocks, 256, 0, st>>>(D, X, n, chunk, w.partial);
-    else k_outer_partial<2><<<blocks, 256, 0, st>>>(D, X, n, chunk, w.partial);
-    kcheck("gnn outer partial");
-    k_partial_final<<<blocks_for(nw + H, 128), 128, 0, st>>>(w.partial, blocks, nw + H, nw, dst_b >= 0 ? H : 0, grad,
-                                                              dst_w, dst_b);
-    kcheck("gnn outer final");
-}
-
-static void wd_grad(const float* coef, const float* X, int n, Work& w, float* grad, int dst_w, int dst_b,
-                    cudaStream_t st) {
-    const int blocks = std::max(1, std::min(kRedBlocks, blocks_for(n, 8)));
-    k_vec_partial<<<blocks, 256, 0, st>>>(coef, X, n, w.partial);
-    kcheck("gnn vec partial");
-    k_partial_final<<<1, 64, 0, st>>>(w.partial, blocks, H + 1, H, 1, grad, dst_w, dst_b);
-    kcheck("gnn vec final");
-}
-
 void loss_backward(const DevGraph& g, const float* wr, Work& w, float* grad, unsigned long long seed, cudaStream_t st) {
     if (w.loss_kind == kLossKaporin) {
         const int n = g.n;
-        const int nodes_blocks = blocks_for(static_cast<long long>(n) * 32, 256);
+        const int nodes_blocks = blocks_for(static_cast<long long>(n) * kNodeLanes, 256);
         kcheck_status(cudaMemsetAsync(w.bad, 0, sizeof(int), st), "gnn memset");
         k_kaporin<<<nodes_blocks, 256, 0, st>>>(g.low_ptr, g.low_col, g.adj_ptr, g.adj_col, g.adj_e, w.go, w.gd, w.td,
                                                 n, 0, w.r, w.dgo, w.dexp, nullptr, nullptr, w.bad);
         kcheck("gnn kaporin");
         const int lb = std::min(kRedBlocks, blocks_for(n, 256));
         k_sum_partial<<<lb, 256, 0, st>>>(w.r, n, w.dpartial);
-        k_dsum_final<<<1, 32, 0, st>>>(w.dpartial, lb, 1.0 / static_cast<double>(n), w.loss);
+        k_dsum_final<<<1, kRedBlocks, 0, st>>>(w.dpartial, lb, 1.0 / static_cast<double>(n), w.loss);
         kcheck("gnn kaporin loss");
         if (grad) backward_from_dg(g, wr, w, grad, st);
         return;
@@ -1286,46 +1425,73 @@ void loss_backward(const DevGraph& g, const float* wr, Work& w, float* grad, uns
 void backward_from_dg(const DevGraph& g, const float* wr, Work& w, float* grad, cudaStream_t st) {
     const ParamOffsets off = param_offsets();
     const int n = g.n;
-    const int nodes_blocks = blocks_for(static_cast<long long>(n) * 32, 256);
+    const int nodes_blocks = blocks_for(static_cast<long long>(n) * kNodeLanes, 256);
     const int lin_blocks = std::min(blocks_for(n, 8 * 16), 148 * 8);  // 8 warps of 16-node tiles
-    k_head_back<<<nodes_blocks, 256, 0, st>>>(g.low_ptr, g.up_ptr, g.up_k, w.zpre, w.dgo, wr, off, w.dph, w.dqh, n);
+    // where each sum's partial rows lie
+    float* next = w.partial;
+    auto rows = [&](int stride) {
+        float* p = next;
+        next += static_cast<size_t>(kGradBlocks) * stride;
+        return p;
+    };
+    GradTable table;
+    // edge head: dph, dqh, and the parameters w, c, c2, bw
+    float* edge = rows(kEdgeRow);
+    k_head_back<<<kGradBlocks, 256, 0, st>>>(g.low_ptr, g.up_ptr, g.up_k, w.zpre, w.dgo, g.low_e, g.low_f, wr, off, w.dph,
+                                             w.dqh, n, edge);
     kcheck("gnn head back");
-    // edge-head parameters w, c, bw
-    {
-        const int eb = std::max(1, std::min(kRedBlocks, blocks_for(g.n_low, 8)));
-        k_edge_partial<<<eb, 256, 0, st>>>(w.zpre, w.dgo, g.low_e, g.low_f, wr, off, g.n_low, w.partial);
-        kcheck("gnn edge partial");
-        // partial rows: [dw (H) | dc (H) | dc2 (H) | dbw (1)]
-        k_partial_final<<<1, 128, 0, st>>>(w.partial, eb, kEdgeRow, H, 0, grad, off.w, -1);
-        k_partial_final<<<1, 128, 0, st>>>(w.partial + H, eb, kEdgeRow, H, 0, grad, off.c, -1);
-        k_partial_final<<<1, 128, 0, st>>>(w.partial + 2 * H, eb, kEdgeRow, H, 0, grad, off.c2, -1);
-        k_partial_final<<<1, 32, 0, st>>>(w.partial + 3 * H, eb, kEdgeRow, 1, 0, grad, off.bw, -1);
-        kcheck("gnn edge final");
-    }
+    table.add(edge, kEdgeRow, H, off.w);
+    table.add(edge + H, kEdgeRow, H, off.c);
+    table.add(edge + 2 * H, kEdgeRow, H, off.c2);
+    table.add(edge + 3 * H, kEdgeRow, 1, off.bw);
+    // dW_m = D_m^T X for up to three matrices of one X; dst_b < 0: no bias
+    auto outer = [&](std::initializer_list<const float*> D, const float* X, std::initializer_list<int> dst_w,
+                     std::initializer_list<int> dst_b) {
+        OuterArgs o{};
+        int m = 0;
+        for (const float* d : D) {
+            o.D[m] = d;
+            o.partial[m] = rows(kOuterRow);
+            table.add(o.partial[m], kOuterRow, H * H, dst_w.begin()[m]);
+            if (dst_b.begin()[m] >= 0) table.add(o.partial[m] + H * H, kOuterRow, H, dst_b.begin()[m]);
+            ++m;
+        }
+        k_outer_partial<<<dim3(kGradBlocks, m), 256, 0, st>>>(o, X, n);
+        kcheck("gnn outer partial");
+    };
     const float* hL = w.h[kLayers];
-    outer_grad(w.dph, hL, H, n, w, grad, off.P, off.bp, st);
-    outer_grad(w.dqh, hL, H, n, w, grad, off.Q, -1, st);
-    // dh = dph P + dqh Q + dexp wd
-    BackLin B{{wr + off.P, wr + off.Q, nullptr}, {w.dph, w.dqh, nullptr}, 2, w.dexp, wr + off.wd, 0};
+    outer({w.dph, w.dqh}, hL, {off.P, off.Q}, {off.bp, -1});
+    // diagonal head: wd, bwd
+    float* diag = rows(H + 1);
+    k_vec_partial<1><<<kGradBlocks, 256, 0, st>>>(w.dexp, hL, n, diag);
+    kcheck("gnn vec partial");
+    table.add(diag, H + 1, H, off.wd);
+    table.add(diag + H, H + 1, 1, off.bwd);
+    // dh = dph P + dqh Q + dexp wd, and ds of the last layer
+    float *ds = w.ds, *ds_next = w.ds2;
+    BackLin B{{wr + off.P, wr + off.Q, nullptr}, {w.dph, w.dqh, nullptr}, 2, w.dexp, wr + off.wd, 0,
+              w.s[kLayers - 1], ds, 1};
     k_node_backlin<<<lin_blocks, 256, 0, st>>>(B, w.dh, n);
     kcheck("gnn head backlin");
-    wd_grad(w.dexp, hL, n, w, grad, off.wd, off.bwd, st);
     for (int l = kLayers - 1; l >= 0; --l) {
-        k_agg_back<<<nodes_blocks, 256, 0, st>>>(g.adj_ptr, g.adj_col, g.adj_e, w.dh, w.s[l], w.ds, w.dhl, w.dhu, n);
+        k_agg_back<<<nodes_blocks, 256, 0, st>>>(g.adj_ptr, g.adj_col, g.adj_e, ds, w.dhl, w.dhu, n);
         kcheck("gnn agg back");
-        const float* hin = w.h[l];
-        outer_grad(w.ds, hin, H, n, w, grad, off.Wa[l], off.ba[l], st);
-        outer_grad(w.dhl, hin, H, n, w, grad, off.Wl[l], -1, st);
-        outer_grad(w.dhu, hin, H, n, w, grad, off.Wu[l], -1, st);
-        // dh <- dh + ds Wa + dhl Wl + dhu Wu
-        BackLin Bl{{wr + off.Wa[l], wr + off.Wl[l], wr + off.Wu[l]}, {w.ds, w.dhl, w.dhu}, 3, nullptr, nullptr, 1};
+        outer({ds, w.dhl, w.dhu}, w.h[l], {off.Wa[l], off.Wl[l], off.Wu[l]}, {off.ba[l], -1, -1});
+        // dh <- dh + ds Wa + dhl Wl + dhu Wu, masked by the layer below (h0 > 0 iff its
+        // pre-activation > 0); below the first layer only the masked form is needed
+        BackLin Bl{{wr + off.Wa[l], wr + off.Wl[l], wr + off.Wu[l]}, {ds, w.dhl, w.dhu}, 3, nullptr, nullptr, 1,
+                   l > 0 ? w.s[l - 1] : w.h[0], ds_next, l > 0 ? 1 : 0};
         k_node_backlin<<<lin_blocks, 256, 0, st>>>(Bl, w.dh, n);
         kcheck("gnn layer backlin");
+        std::swap(ds, ds_next);
     }
-    k_relu_mask<<<blocks_for(static_cast<long long>(n) * H, 256), 256, 0, st>>>(w.dh, w.h[0], w.dh2,
-                                                                              static_cast<long long>(n) * H);
-    kcheck("gnn input mask");
-    outer_grad(w.dh2, g.x, 2, n, w, grad, off.W0, off.b0, st);
+    float* input = rows(3 * H);
+    k_vec_partial<2><<<kGradBlocks, 256, 0, st>>>(g.x, ds, n, input);
+    kcheck("gnn input partial");
+    table.add(input, 3 * H, 2 * H, off.W0);
+    table.add(input + 2 * H, 3 * H, H, off.b0);
+    k_grad_final<<<table.blocks(), 256, 0, st>>>(table, grad);
+    kcheck("gnn gradient sums");
 }
 
 void adam_step(float* theta, const float* grad, float* m, float* v, int P, float lr, int step, cudaStream_t st) {

@@ -74,7 +74,7 @@ struct Work {
     int* bad = nullptr;
     float *v = nullptr, *w1 = nullptr, *w2 = nullptr, *r = nullptr, *t = nullptr, *y = nullptr;
     float *dgo = nullptr, *dexp = nullptr;
-    float *dh = nullptr, *dh2 = nullptr, *ds = nullptr, *dhl = nullptr, *dhu = nullptr, *dph = nullptr, *dqh = nullptr;
+    float *dh = nullptr, *ds2 = nullptr, *ds = nullptr, *dhl = nullptr, *dhu = nullptr, *dph = nullptr, *dqh = nullptr;
     float* partial = nullptr;
     double* dpartial = nullptr;
     double* loss = nullptr;
