@@ -412,6 +412,13 @@ __device__ __forceinline__ void undefine(float2& x) { undefine(x.x); undefine(x.
 __device__ __forceinline__ void undefine(uint2& x) { undefine(x.x); undefine(x.y); }
 __device__ __forceinline__ void undefine(float4& x) { undefine(x.x); undefine(x.y); undefine(x.z); undefine(x.w); }
 
+// threadIdx.x read anew: nothing derived from it is kept in registers from an earlier use.
+__device__ __forceinline__ int thread_index() {
+    int t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
+}
+
 template <typename VT, int CHUNK, int DEPTH>
 struct SlotRing {
     using RV = typename RawVec<typename RawOf<VT>::type, CHUNK>::type;
@@ -472,6 +479,47 @@ struct SlotRing {
                     undefine(c[j][k][h]);
                 }
             fetch(j);
+        }
+    }
+    // prime() that writes every register of the ring on every path (a chunk beyond its slice repeats
+    // the last one, a slice that is not there gives zeros; neither is used).  A register that keeps
+    // its old value on some path is live from one iteration's run() to the next one's prime(), which
+    // a kernel with other large users of registers in between cannot afford.
+    __device__ __forceinline__ void prime_all(int warp) {
+        ls = sb + warp;
+        lc = 0;
+#pragma unroll
+        for (int j = 0; j < DEPTH; ++j) {
+            int wmax = 0;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int s = ls + k * wpb;
+                const int2 sl = s < se ? table[s - sb] : make_int2(0, 0);
+                wmax = max(wmax, sl.y);
+                if (lc < sl.y) {
+                    const bool staged = s < sm_end;
+                    const int off = sl.x - (staged ? m0 : 0) + lane * CHUNK;
+                    const VT* vp = (staged ? mval : val) + off;
+                    const short* cp = (staged ? mcol : col) + off;
+#pragma unroll
+                    for (int h = 0; h < HC; ++h) {
+                        const int at = min(lc + h * CHUNK, sl.y - CHUNK) * 32;
+                        v[j][k][h] = *reinterpret_cast<const RV*>(vp + at);
+                        c[j][k][h] = *reinterpret_cast<const RC*>(cp + at);
+                    }
+                } else {
+#pragma unroll
+                    for (int h = 0; h < HC; ++h) {
+                        v[j][k][h] = RV{};
+                        c[j][k][h] = RC{};
+                    }
+                }
+            }
+            lc += kUnit;
+            if (lc >= wmax) {
+                ls += 2 * wpb;
+                lc = 0;
+            }
         }
     }
     // Products of the primed band with the window pw (row w0 first): row_done(row, p'_row, y) for

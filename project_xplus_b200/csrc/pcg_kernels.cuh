@@ -39,6 +39,7 @@ struct PcgArgs {
     // optional M^-1 = G^T G (G and its transpose in SELL form over the same ordering)
     const long long* g_slice_ptr; const int* g_col; const void* g_val;
     const long long* gt_slice_ptr; const int* gt_col; const void* gt_val;
+    const short* g_col16; const short* gt_col16;  // SM-resident form: offsets from the row
     void* t;                // XT, n_pad: G r temporary
     void* z;                // XT, n_pad: preconditioned residual (GTG mode only)
     double* partial;        // 2 banks x 4 slots x gridDim.x
@@ -109,6 +110,19 @@ cudaError_t resident_launch(const KernelKey& k, const PcgArgs& a, int grid, int 
 cudaError_t gtg_grid(const KernelKey& k, int device, int n_slices, int* grid, int* tpb);
 cudaError_t gtg_launch(const KernelKey& k, const PcgArgs& a, int grid, int tpb, cudaStream_t s,
                        const cudaAccessPolicyWindow& window);
+// SM-resident GTG kernel (pcg_gtg_resident.cu): the same iteration for systems whose bands, with the
+// windows of p', r' and t, fit shared memory at the grid of gtg_grid.
+constexpr int kGtgResSlices = 256;  // slice table capacity per CTA
+bool gtg_res_supported(const KernelKey& k);
+size_t gtg_res_vector_bytes(int rows, int window);
+cudaError_t gtg_res_prepare(const KernelKey& k, int device, size_t vector_bytes, size_t matrix_bytes, bool* fits,
+                            size_t* smem_bytes);
+cudaError_t gtg_res_launch(const KernelKey& k, const PcgArgs& a, int grid, size_t smem_bytes, cudaStream_t s);
+// int16 offsets of a G or G^T image (chunk 2, |col - row| < 32768), and per block of `grid` the window
+// {first row, rows} that the columns of A (int16 offsets) reach, widened to multiples of 4
+cudaError_t gtg_pack16(const long long* slice_ptr, int n_slices, const int* col, short* col16, cudaStream_t s);
+cudaError_t gtg_windows(const long long* slice_ptr, const short* col16, int chunk, int n_slices, int n_pad, int grid,
+                        int2* win, cudaStream_t s);
 // val[q] = glow[map[q]] (0 where map[q] < 0): G values into a SELL image of G or G^T
 cudaError_t gtg_fill_values(const double* d_glow, const int* d_map, float* d_val, long long slots, cudaStream_t s);
 cudaError_t spmv_launch(const KernelKey& k, const SpmvArgs& a, const void* x, void* y,

@@ -87,6 +87,10 @@ struct xplus_pcg {
     int *d_g_col = nullptr, *d_gt_col = nullptr, *d_g_map = nullptr, *d_gt_map = nullptr;
     float *d_g_val = nullptr, *d_gt_val = nullptr, *d_t = nullptr, *d_r2 = nullptr;
     double* d_glow = nullptr;
+    bool gtg_res = false;      // its SM-resident form (pcg_gtg_resident.cu)
+    size_t gtg_smem = 0;
+    short *d_g_col16 = nullptr, *d_gt_col16 = nullptr;
+    int2* d_gtg_win = nullptr;
 };
 
 namespace xplus {
@@ -719,7 +723,15 @@ void enqueue_solve(xplus_pcg* h, double tau, int tau_mode, int max_iters_in, int
         a.t = h->d_t;
         a.r2 = h->d_r2;
         a.g_fallback_iters = h->g_fallback_iters;
-        cuda_check(gtg_launch(h->key, a, h->gtg_grid, 512, st, h->window), "GTG PCG launch");
+        if (h->gtg_res) {
+            a.g_col16 = h->d_g_col16;
+            a.gt_col16 = h->d_gt_col16;
+            a.win = h->d_gtg_win;
+            a.smem_bytes = static_cast<int>(h->gtg_smem);
+            a.z = h->d_rec;
+            cuda_check(gtg_res_launch(h->key, a, h->gtg_grid, h->gtg_smem, st), "resident GTG PCG launch");
+        } else
+            cuda_check(gtg_launch(h->key, a, h->gtg_grid, 512, st, h->window), "GTG PCG launch");
     } else if (h->resident)
         // no access-policy window: the resident kernel's only global stream is a matrix that L2
         // holds anyway, and the launch attribute cost time (1108^2 system: 97.1 ms with it,
@@ -839,6 +851,45 @@ void gtg_layout_host(xplus_pcg* h, const int* row_ptr, const int* col_idx) {
     cuda_check(cudaStreamSynchronize(st), "sync");  // the host images go next
 }
 
+// The SM-resident G^T G kernel, when the handle's bands fit it: windows, int16 offsets of G and G^T
+// (their patterns lie within A's, whose offsets are int16), shared memory.
+void gtg_resident(xplus_pcg* h) {
+    const int grid = h->gtg_grid, per = (h->n_slices + grid - 1) / grid;
+    if (!gtg_res_supported(h->key) || !h->opts.resident || per > kGtgResSlices) return;
+    cudaStream_t st = h->stream;
+    h->d_gtg_win = dalloc<int2>(h, static_cast<size_t>(grid));
+    cuda_check(gtg_windows(h->d_slice_ptr, static_cast<const short*>(h->d_col), h->opts.chunk, h->n_slices, h->n_pad, grid,
+                           h->d_gtg_win, st), "gtg windows");
+    const int bands = (h->n_slices + per - 1) / per;
+    std::vector<int2> win(static_cast<size_t>(grid));
+    cuda_check(cudaMemcpyAsync(win.data(), h->d_gtg_win, win.size() * sizeof(int2), cudaMemcpyDeviceToHost, st), "D2H");
+    // first slots of the bands in A, G and G^T
+    const long long* sp[3] = {h->d_slice_ptr, h->d_g_slice_ptr, h->d_gt_slice_ptr};
+    const long long total[3] = {h->slots, h->g_slots, h->gt_slots};
+    std::vector<long long> bp[3];
+    for (int m = 0; m < 3; ++m) {
+        bp[m].resize(static_cast<size_t>(bands) + 1);
+        cuda_check(cudaMemcpy2DAsync(bp[m].data(), sizeof(long long), sp[m], static_cast<size_t>(per) * sizeof(long long),
+                                     sizeof(long long), static_cast<size_t>(bands), cudaMemcpyDeviceToHost, st), "D2H");
+        bp[m][static_cast<size_t>(bands)] = total[m];
+    }
+    cuda_check(cudaStreamSynchronize(st), "sync");
+    size_t vec = 0;
+    long long mat = 0;
+    for (int b = 0; b < bands; ++b) {
+        const size_t k = static_cast<size_t>(b);
+        vec = std::max(vec, gtg_res_vector_bytes((std::min(h->n_slices, (b + 1) * per) - b * per) * 32, win[k].y));
+        mat = std::max(mat, (bp[0][k + 1] - bp[0][k]) * static_cast<long long>(elem_size(h->opts.value_type) + 2) +
+                                (bp[1][k + 1] - bp[1][k] + bp[2][k + 1] - bp[2][k]) * 6);
+    }
+    cuda_check(gtg_res_prepare(h->key, h->device, vec, static_cast<size_t>(mat), &h->gtg_res, &h->gtg_smem), "gtg resident");
+    if (!h->gtg_res) return;
+    h->d_g_col16 = dalloc<short>(h, static_cast<size_t>(h->g_slots));
+    h->d_gt_col16 = dalloc<short>(h, static_cast<size_t>(h->gt_slots));
+    cuda_check(gtg_pack16(h->d_g_slice_ptr, h->n_slices, h->d_g_col, h->d_g_col16, st), "gtg pack");
+    cuda_check(gtg_pack16(h->d_gt_slice_ptr, h->n_slices, h->d_gt_col, h->d_gt_col16, st), "gtg pack");
+}
+
 // The G / G^T images and the vectors of the G^T G kernel for the pattern of the CSR given to
 // xplus_pcg_create (once per handle): on the GPU unless the handle was built on the host.
 void gtg_layout(xplus_pcg* h, const int* row_ptr, const int* col_idx) {
@@ -880,6 +931,7 @@ void gtg_layout(xplus_pcg* h, const int* row_ptr, const int* col_idx) {
         h->d_partial = dalloc<double>(h, static_cast<size_t>(16) * h->gtg_grid);
         h->d_block_clk = dalloc<long long>(h, static_cast<size_t>(4) * h->gtg_grid);
     }
+    gtg_resident(h);
     cuda_check(cudaStreamSynchronize(st), "sync");
 }
 
@@ -891,7 +943,7 @@ void gtg_enable(xplus_pcg* h, int fallback_iters) {
     cuda_check(cudaStreamSynchronize(st), "sync");
     h->g_fallback_iters = fallback_iters;
     h->gtg = true;
-    request_l2(h);
+    if (!h->gtg_res) request_l2(h);
 }
 
 }  // namespace
