@@ -43,8 +43,8 @@ struct PcgArgs {
     void* t;                // XT, n_pad: G r temporary
     void* z;                // XT, n_pad: preconditioned residual (GTG mode only)
     double* partial;        // 2 banks x 4 slots x gridDim.x
-    int smem_bytes;         // one-barrier SM-resident kernel: its dynamic shared memory (what the
-                            // vectors leave holds matrix slots)
+    int smem_bytes;         // dynamic shared memory of the launch, for the kernels that keep matrix
+                            // slots in what their vectors leave of it
     unsigned* bar;
     int* err;
     PcgOut* out;
@@ -105,6 +105,11 @@ cudaError_t resident_prepare(const KernelKey& k, int device, size_t vector_bytes
                              bool one_sync, bool* fits, size_t* smem_bytes);
 cudaError_t resident_launch(const KernelKey& k, const PcgArgs& a, int grid, int tpb, size_t smem_bytes,
                             bool one_sync, cudaStream_t s, const cudaAccessPolicyWindow& window);
+// One-CTA kernel for FP64 vectors (pcg_small.cu): pcg_persistent_kernel's solve for systems of at most
+// four slices per warp.
+cudaError_t small_prepare(const KernelKey& k, int device, int n_slices, long long matrix_bytes, int tpb, bool* fits,
+                          size_t* smem_bytes);
+cudaError_t small_launch(const KernelKey& k, const PcgArgs& a, int tpb, size_t smem_bytes, cudaStream_t s);
 // GTG-preconditioned persistent kernel (pcg_gtg.cu): FP32 vectors, row-sum form, M^-1 = G^T G
 // with G and G^T in SELL form (FP32 values, int32 columns, chunk 2) over the matrix's ordering.
 cudaError_t gtg_grid(const KernelKey& k, int device, int n_slices, int* grid, int* tpb);

@@ -63,6 +63,7 @@ struct xplus_pcg {
     int grid = 0, tpb = 0;
     bool resident = false;     // SM-resident kernel (pcg_resident.cu)
     bool one_sync = false;     // its one-barrier-per-iteration form
+    bool small = false;        // one-CTA kernel (pcg_small.cu)
     double val_scale = 1.0;    // stored value = a_ij / val_scale (FP16)
     size_t smem_bytes = 0;
     int2* d_win = nullptr;
@@ -632,7 +633,11 @@ void create(const int* row_ptr, const int* col_idx, const double* values, int n,
         }
         if (!h->resident) {
             cuda_check(pcg_grid(h->key, o.device, h->n_slices, want_tpb, o.blocks_per_sm, &h->grid, &h->tpb), "pcg_grid");
-            request_l2(h);
+            if (h->grid == 1)
+                cuda_check(small_prepare(h->key, o.device, h->n_slices,
+                                         h->slots * static_cast<long long>(elem_size(o.value_type) + (h->key.idx16 ? 2 : 4)),
+                                         h->tpb, &h->small, &h->smem_bytes), "small_prepare");
+            if (!h->small) request_l2(h);
         }
         h->d_partial = dalloc<double>(h, static_cast<size_t>(16) * h->grid);
         // barrier counter, error flag and outcome: one block, zeroed by one memset
@@ -739,6 +744,8 @@ void enqueue_solve(xplus_pcg* h, double tau, int tau_mode, int max_iters_in, int
         cuda_check(resident_launch(h->key, a, h->grid, h->tpb, h->smem_bytes, h->one_sync, st,
                                    cudaAccessPolicyWindow{}),
                    "resident PCG launch");
+    else if (h->small && h->debug_skip_block < 0)
+        cuda_check(small_launch(h->key, a, h->tpb, h->smem_bytes, st), "one-CTA PCG launch");
     else
         cuda_check(pcg_launch(h->key, a, h->grid, h->tpb, st, h->window), "persistent PCG launch");
     cuda_check(cudaEventRecord(h->ev1, st), "event");
@@ -748,10 +755,12 @@ void enqueue_solve(xplus_pcg* h, double tau, int tau_mode, int max_iters_in, int
 void collect(xplus_pcg* h, xplus_metrics* m) {
     if (h->pending) {
         cuda_check(cudaEventSynchronize(h->ev1), "sync");
+        unsigned char ctl[kCtlBytes];
+        cuda_check(cudaMemcpy(ctl, h->d_ctl, kCtlBytes, cudaMemcpyDeviceToHost), "D2H");
         PcgOut o{};
         int err = 0;
-        cuda_check(cudaMemcpy(&o, h->d_out, sizeof(PcgOut), cudaMemcpyDeviceToHost), "D2H");
-        cuda_check(cudaMemcpy(&err, h->d_err, sizeof(int), cudaMemcpyDeviceToHost), "D2H");
+        std::memcpy(&o, ctl + 256, sizeof(PcgOut));
+        std::memcpy(&err, ctl + 128, sizeof(int));
         float ms = 0.0f;
         cuda_check(cudaEventElapsedTime(&ms, h->ev0, h->ev1), "event");
         xplus_metrics& L = h->last;
