@@ -419,7 +419,8 @@ __device__ __forceinline__ int thread_index() {
     return t;
 }
 
-template <typename VT, int CHUNK, int DEPTH>
+// STREAM: the slots (none of them in shared memory) are read past L1 and are the first to leave L2.
+template <typename VT, int CHUNK, int DEPTH, bool STREAM = false>
 struct SlotRing {
     using RV = typename RawVec<typename RawOf<VT>::type, CHUNK>::type;
     using RC = typename RawVec<unsigned short, CHUNK>::type;
@@ -455,8 +456,13 @@ struct SlotRing {
 #pragma unroll
                 for (int h = 0; h < HC; ++h)
                     if (lc + h * CHUNK < sl.y) {
-                        v[j][k][h] = *reinterpret_cast<const RV*>(vp + h * 32 * CHUNK);
-                        c[j][k][h] = *reinterpret_cast<const RC*>(cp + h * 32 * CHUNK);
+                        if constexpr (STREAM) {
+                            v[j][k][h] = ld_na(reinterpret_cast<const RV*>(vp + h * 32 * CHUNK));
+                            c[j][k][h] = ld_na(reinterpret_cast<const RC*>(cp + h * 32 * CHUNK));
+                        } else {
+                            v[j][k][h] = *reinterpret_cast<const RV*>(vp + h * 32 * CHUNK);
+                            c[j][k][h] = *reinterpret_cast<const RC*>(cp + h * 32 * CHUNK);
+                        }
                     }
             }
         }

@@ -105,6 +105,11 @@ cudaError_t resident_prepare(const KernelKey& k, int device, size_t vector_bytes
                              bool one_sync, bool* fits, size_t* smem_bytes);
 cudaError_t resident_launch(const KernelKey& k, const PcgArgs& a, int grid, int tpb, size_t smem_bytes,
                             bool one_sync, cudaStream_t s, const cudaAccessPolicyWindow& window);
+// The global-memory kernel's solve with the window of p' in shared memory (pcg_window.cu): FP32 vectors,
+// row-sum form, int16 offsets, at pcg_grid's grid; a.win: its blocks' windows.
+cudaError_t window_prepare(const KernelKey& k, int device, int n_slices, int grid, int tpb, int window, bool* fits,
+                           size_t* smem_bytes);
+cudaError_t window_launch(const KernelKey& k, const PcgArgs& a, int grid, int tpb, size_t smem_bytes, cudaStream_t s);
 // One-CTA kernel for FP64 vectors (pcg_small.cu): pcg_persistent_kernel's solve for systems of at most
 // four slices per warp.
 cudaError_t small_prepare(const KernelKey& k, int device, int n_slices, long long matrix_bytes, int tpb, bool* fits,

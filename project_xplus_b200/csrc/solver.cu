@@ -64,6 +64,7 @@ struct xplus_pcg {
     bool resident = false;     // SM-resident kernel (pcg_resident.cu)
     bool one_sync = false;     // its one-barrier-per-iteration form
     bool small = false;        // one-CTA kernel (pcg_small.cu)
+    bool windowed = false;     // p' window in shared memory, the rest in global (pcg_window.cu)
     double val_scale = 1.0;    // stored value = a_ij / val_scale (FP16)
     size_t smem_bytes = 0;
     int2* d_win = nullptr;
@@ -637,7 +638,18 @@ void create(const int* row_ptr, const int* col_idx, const double* values, int n,
                 cuda_check(small_prepare(h->key, o.device, h->n_slices,
                                          h->slots * static_cast<long long>(elem_size(o.value_type) + (h->key.idx16 ? 2 : 4)),
                                          h->tpb, &h->small, &h->smem_bytes), "small_prepare");
-            if (!h->small) request_l2(h);
+            // the windows were made for one block per SM: the grid of a system this large
+            if (h->grid == res_grid && static_cast<int>(win.size()) == res_grid) {
+                int max_wn = 0;
+                for (const int2& w : win) max_wn = std::max(max_wn, w.y);
+                cuda_check(window_prepare(h->key, o.device, h->n_slices, h->grid, h->tpb, max_wn, &h->windowed,
+                                          &h->smem_bytes), "window_prepare");
+                if (h->windowed) {
+                    h->d_win = dalloc<int2>(h, win.size());
+                    cuda_check(cudaMemcpyAsync(h->d_win, win.data(), win.size() * sizeof(int2), cudaMemcpyHostToDevice, st), "H2D");
+                }
+            }
+            if (!h->small && !h->windowed) request_l2(h);
         }
         h->d_partial = dalloc<double>(h, static_cast<size_t>(16) * h->grid);
         // barrier counter, error flag and outcome: one block, zeroed by one memset
@@ -744,6 +756,8 @@ void enqueue_solve(xplus_pcg* h, double tau, int tau_mode, int max_iters_in, int
         cuda_check(resident_launch(h->key, a, h->grid, h->tpb, h->smem_bytes, h->one_sync, st,
                                    cudaAccessPolicyWindow{}),
                    "resident PCG launch");
+    else if (h->windowed)
+        cuda_check(window_launch(h->key, a, h->grid, h->tpb, h->smem_bytes, st), "windowed PCG launch");
     else if (h->small && h->debug_skip_block < 0)
         cuda_check(small_launch(h->key, a, h->tpb, h->smem_bytes, st), "one-CTA PCG launch");
     else
