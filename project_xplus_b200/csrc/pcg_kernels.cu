@@ -341,10 +341,11 @@ __global__ void gather_kernel(const double* __restrict__ src, T* __restrict__ ds
     if (i < n_pad) dst[i] = i < n ? static_cast<T>(src[perm[i]]) : T(0);
 }
 
-__global__ void scatter_kernel(const double* __restrict__ src, double* __restrict__ dst,
+template <typename T>
+__global__ void scatter_kernel(const T* __restrict__ src, double* __restrict__ dst,
                                const int* __restrict__ perm, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[perm[i]] = src[i];
+    if (i < n) dst[perm[i]] = static_cast<double>(src[i]);
 }
 
 // ---- dispatch over (value type, vector type, chunk, row-sum form, index width) ----
@@ -482,11 +483,18 @@ cudaError_t gather_to_sell(int xt, const double* src, void* dst, const int* perm
     return cudaGetLastError();
 }
 
+cudaError_t scatter_widened(int xt, const void* src, double* dst, const int* perm, int n, cudaStream_t s) {
+    const int threads = 256, blocks = (n + threads - 1) / threads;
+    if (xt == XPLUS_F32)
+        scatter_kernel<<<blocks, threads, 0, s>>>(static_cast<const float*>(src), dst, perm, n);
+    else
+        scatter_kernel<<<blocks, threads, 0, s>>>(static_cast<const double*>(src), dst, perm, n);
+    return cudaGetLastError();
+}
+
 cudaError_t scatter_from_sell(const double* src, double* dst, const int* perm, int n,
                               cudaStream_t s) {
-    const int threads = 256, blocks = (n + threads - 1) / threads;
-    scatter_kernel<<<blocks, threads, 0, s>>>(src, dst, perm, n);
-    return cudaGetLastError();
+    return scatter_widened(XPLUS_F64, src, dst, perm, n, s);
 }
 
 }  // namespace xplus

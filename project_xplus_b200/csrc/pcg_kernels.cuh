@@ -140,6 +140,8 @@ cudaError_t spmv_launch(const KernelKey& k, const SpmvArgs& a, const void* x, vo
 // dst[i] = (T) src[perm[i]] for i < n, 0 for n <= i < n_pad   (T per xt; f64 when xt==F64)
 cudaError_t gather_to_sell(int xt, const double* src, void* dst, const int* perm, int n, int n_pad,
                            cudaStream_t s);
+// dst[perm[i]] = (double) src[i], src of the vector type xt
+cudaError_t scatter_widened(int xt, const void* src, double* dst, const int* perm, int n, cudaStream_t s);
 // dst[perm[i]] = src[i]
 cudaError_t scatter_from_sell(const double* src, double* dst, const int* perm, int n,
                               cudaStream_t s);

@@ -1136,17 +1136,10 @@ int xplus_pcg_spmv(xplus_pcg* h, const double* x, double* y) {
         SpmvArgs a{h->n_pad, h->n_slices, h->d_slice_ptr, h->d_col, h->d_val, h->d_rowsum,
                    static_cast<float>(h->val_scale)};
         cuda_check(spmv_launch(h->key, a, h->d_sx, h->d_sy, st), "spmv");
-        // widen the SELL-order result to FP64 and scatter to original order
-        std::vector<unsigned char> ys(static_cast<size_t>(h->n_pad) * elem_size(h->opts.vector_type));
-        cuda_check(cudaMemcpyAsync(ys.data(), h->d_sy, ys.size(), cudaMemcpyDeviceToHost, st), "D2H");
-        std::vector<int> perm(static_cast<size_t>(h->n));
-        cuda_check(cudaMemcpyAsync(perm.data(), h->d_perm, perm.size() * sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
+        // the result widened to FP64 in original order, through the staging vector (its x has been read)
+        cuda_check(scatter_widened(h->opts.vector_type, h->d_sy, h->d_xio, h->d_perm, h->n, st), "scatter");
+        cuda_check(cudaMemcpyAsync(y, h->d_xio, nb, cudaMemcpyDeviceToHost, st), "D2H");
         cuda_check(cudaStreamSynchronize(st), "sync");
-        for (int i = 0; i < h->n; ++i) {
-            const double v = h->opts.vector_type == XPLUS_F64 ? reinterpret_cast<double*>(ys.data())[i]
-                                                              : static_cast<double>(reinterpret_cast<float*>(ys.data())[i]);
-            y[perm[static_cast<size_t>(i)]] = v;
-        }
     });
 }
 
