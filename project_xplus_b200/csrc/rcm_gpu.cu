@@ -7,15 +7,25 @@
 // The GPU computes the same order level by level.  When the nodes of level L sit at queue
 // positions [lb, le), the host gives each node u of level L + 1 to the first node of level L
 // (lowest position) adjacent to it, and lists level L + 1 parent by parent, each parent's
-// children by (degree, index).  So one persistent cooperative launch per BFS does, per level:
-//   claim   every unvisited neighbour u of frontier node p: claim[u] = min(claim[u], p)
-//   count   children of p = #{u in adj(p) : claim[u] == p}
-//   write   exclusive scan of the counts in frontier order gives every parent its offset;
-//           it writes its children sorted by (degree, index) there
-// with a bounded grid barrier between the steps.  The pseudo-peripheral search uses the same
-// BFS (only its level count and last level matter there).  A node with more than kMaxChildren
-// claimed children, or a row with a repeated column, sends the whole ordering to the host
-// function instead (same result, host speed).
+// children by (degree, index).  So the ordering's BFS (k_bfs, one persistent cooperative launch)
+// does, per level:
+//   count   children of p = {u in adj(p) : claim[u] == p}, kept in shared memory
+//   write   exclusive scan of the counts in frontier order gives every parent its offset; it
+//           writes its children sorted by (degree, index) there, and every child, now that it
+//           has a position, claims its neighbours: claim[w] = min(claim[w], position)
+// with a bounded grid barrier after each.  Positions only grow, so a claim never takes a node
+// that is already in the queue, and the claim array is also the mark of what has been reached.
+// The pseudo-peripheral search needs the level sets alone, in no order: its BFS (k_levels) appends
+// what it reaches through a counter, one grid barrier per level.  A node with more than
+// kMaxChildren claimed children, or a row with a repeated column, sends the whole ordering to the
+// host function instead (same result, host speed).
+//
+// What bounds both is the chain of dependent L2 round trips and barriers of a level (order, row
+// pointers, columns, claims): a level of a 2D mesh of n nodes has about sqrt(n) of them.  Eight
+// lanes take a node, so that a row's columns, and their claims, come in one round trip each.
+// One BFS for both purposes, a thread per node and three barriers per level, with serial sums over
+// the CTAs between them, took rcm_device + permute_symmetric_device of a permuted 500^2 mesh 66.8 ms;
+// this takes 31.1, most of the rest the host's copies and structure checks.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,135 +48,206 @@ constexpr int kFree = 0x7F7F7F7F;  // claim of a node no frontier node has claim
 constexpr int kMaxChildren = 64;
 constexpr int kBfsThreads = 512;
 
+constexpr int kLanes = 8;  // lanes per node
+constexpr int kGroups = kBfsThreads / kLanes;
+
 struct BfsArgs {
     const int* rp;
     const int* ci;
     const int* deg;
-    const int* placed;  // 1: ordered by an earlier component
-    int* vis;           // == stamp: reached by this BFS
-    int* claim;         // kFree, or the lowest frontier position that reached the node
+    int* claim;         // kFree; -1: ordered by an earlier component; else reached (position of the claimant)
     int* order;         // BFS order
-    int* cnt;           // children of each frontier node (frontier-relative)
+    int* cnt;           // children of each frontier node (frontier-relative), where they are counted twice
     int* block_sum;     // per CTA
     int* out;           // {visited, levels, first position of the last level, too many children}
-    int stamp;
+    int* tail;          // k_levels: nodes appended by a level, three levels in turn
     int root;
     unsigned* bar;
     int* err;
     long long timeout_ns;
 };
 
-__device__ __forceinline__ bool before(const int* deg, int a, int b) {
-    const int da = deg[a], db = deg[b];
-    return da < db || (da == db && a < b);
+// What the host reads, and the claims of this BFS taken back.  Every CTA calls it after a barrier.
+__device__ __forceinline__ void finish_bfs(const BfsArgs& a, int visited, int levels, int last_b) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < visited; q += gridDim.x * blockDim.x)
+        a.claim[a.order[q]] = kFree;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.out[0] = visited;
+        a.out[1] = levels;
+        a.out[2] = last_b;
+    }
 }
 
-__global__ void __launch_bounds__(kBfsThreads) k_bfs(BfsArgs a) {
+// Level sets alone: the order of the nodes within a level is whatever the appends make it.
+__global__ void __launch_bounds__(kBfsThreads, 1) k_levels(BfsArgs a) {
     __shared__ int s_flag;
-    __shared__ int s_scan[kBfsThreads];
-    __shared__ int s_run;
     GridBarrier bar{a.bar, a.err, a.timeout_ns, 0u, -1};
+    const int lane = threadIdx.x & 31, l = threadIdx.x & (kLanes - 1);
+    // consecutive warps of a frontier on different SMs
+    const int warp = static_cast<int>((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+    const int warps = static_cast<int>(gridDim.x * (blockDim.x >> 5));
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.order[0] = a.root;
-        a.vis[a.root] = a.stamp;
+        a.claim[a.root] = 0;
     }
     if (!bar.sync(&s_flag)) return;
     int lb = 0, le = 1, levels = 0, last_b = 0;
-    const int gthreads = gridDim.x * blockDim.x;
+    while (le > lb) {
+        int* tail = a.tail + levels % 3;
+        // the next level's counter: its last reading (two levels ago) is a barrier behind
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.tail[(levels + 1) % 3] = 0;
+        ++levels;
+        last_b = lb;
+        const int fs = le - lb;
+        for (int q0 = warp * (32 / kLanes); q0 < fs; q0 += warps * (32 / kLanes)) {
+            const int q = q0 + lane / kLanes;
+            int k = 0, e = 0;
+            if (q < fs) {
+                const int x = a.order[lb + q];
+                k = a.rp[x] + l;
+                e = a.rp[x + 1];
+            }
+            while (__any_sync(0xffffffffu, k < e)) {
+                int u = 0;
+                bool own = false;
+                if (k < e) {
+                    u = a.ci[k];
+                    // a stale kFree only leads to the exchange, which decides
+                    own = a.claim[u] == kFree && atomicCAS(&a.claim[u], kFree, 0) == kFree;
+                }
+                const unsigned got = __ballot_sync(0xffffffffu, own);
+                if (got) {
+                    const int first = __ffs(got) - 1;
+                    int base = 0;
+                    if (lane == first) base = atomicAdd(tail, __popc(got));
+                    base = __shfl_sync(0xffffffffu, base, first);
+                    if (own) a.order[le + base + __popc(got & ((1u << lane) - 1u))] = u;
+                }
+                k += kLanes;
+            }
+        }
+        if (!bar.sync(&s_flag)) return;
+        lb = le;
+        le += ld_volatile_int(tail);
+    }
+    finish_bfs(a, le, levels, last_b);
+}
+
+// The children of frontier node x at position p, as (degree, index) keys, in the group's slots:
+// returns how many there are (those beyond kMaxChildren are counted, not kept).
+__device__ __forceinline__ int gather_children(const BfsArgs& a, int x, int p, unsigned gmask, int l,
+                                               unsigned long long* kid) {
+    int m = 0;
+    const int e = a.rp[x + 1];
+    for (int k0 = a.rp[x]; k0 < e; k0 += kLanes) {
+        const int k = k0 + l;
+        const int u = k < e ? a.ci[k] : -1;
+        const bool own = u >= 0 && u != x && a.claim[u] == p;
+        const unsigned got = (__ballot_sync(gmask, own) & gmask) >> (threadIdx.x & 24);
+        const int at = m + __popc(got & ((1u << l) - 1u));
+        if (own && at < kMaxChildren)
+            kid[at] = (static_cast<unsigned long long>(a.deg[u]) << 32) | static_cast<unsigned>(u);
+        m += __popc(got);
+    }
+    __syncwarp(gmask);
+    return m;
+}
+
+// Cuthill-McKee order from the root.
+__global__ void __launch_bounds__(kBfsThreads, 1) k_bfs(BfsArgs a) {
+    __shared__ int s_flag;
+    __shared__ int s_warp[kBfsThreads / 32];
+    __shared__ int s_cnt[kGroups];
+    __shared__ unsigned long long s_kid[kGroups][kMaxChildren];
+    GridBarrier bar{a.bar, a.err, a.timeout_ns, 0u, -1};
+    const int lane = threadIdx.x & 31, l = threadIdx.x & (kLanes - 1), g = threadIdx.x / kLanes;
+    const unsigned gmask = 0xFFu << (threadIdx.x & 24);
+    unsigned long long* kid = s_kid[g];
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) {
+            a.order[0] = a.root;
+            a.claim[a.root] = -1;
+        }
+        for (int k = a.rp[a.root] + threadIdx.x; k < a.rp[a.root + 1]; k += blockDim.x)
+            if (a.ci[k] != a.root) atomicMin(&a.claim[a.ci[k]], 0);
+    }
+    if (!bar.sync(&s_flag)) return;
+    int lb = 0, le = 1, levels = 0, last_b = 0;
     while (le > lb) {
         ++levels;
         last_b = lb;
         const int fs = le - lb;
-        // claim
-        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < fs; q += gthreads) {
-            const int p = lb + q, x = a.order[p];
-            for (int k = a.rp[x]; k < a.rp[x + 1]; ++k) {
-                const int u = a.ci[k];
-                if (u != x && !a.placed[u] && a.vis[u] != a.stamp) atomicMin(&a.claim[u], p);
-            }
-        }
-        if (!bar.sync(&s_flag)) return;
-        // count, over contiguous frontier chunks per CTA
+        // count, over contiguous frontier chunks per CTA; a chunk of one node per group keeps its children
         const int chunk = (fs + gridDim.x - 1) / gridDim.x;
         const int c0 = min(fs, static_cast<int>(blockIdx.x) * chunk), c1 = min(fs, c0 + chunk);
-        int mine = 0;
-        for (int q = c0 + threadIdx.x; q < c1; q += blockDim.x) {
-            const int p = lb + q, x = a.order[p];
-            int c = 0;
-            for (int k = a.rp[x]; k < a.rp[x + 1]; ++k) {
-                const int u = a.ci[k];
-                c += (u != x && a.claim[u] == p);
+        const bool held = chunk <= kGroups;
+        int mine = 0, m = 0;
+        for (int q = c0 + g; q < c1; q += kGroups) {
+            m = gather_children(a, a.order[lb + q], lb + q, gmask, l, kid);
+            if (l == 0) {
+                if (m > kMaxChildren) atomicExch(a.out + 3, 1);
+                if (!held) a.cnt[q] = m;
+                mine += m;
             }
-            if (c > kMaxChildren) atomicExch(a.out + 3, 1);
-            a.cnt[q] = c;
-            mine += c;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-        if ((threadIdx.x & 31) == 0) s_scan[threadIdx.x >> 5] = mine;
+        __syncwarp();
+        mine = __reduce_add_sync(0xffffffffu, mine);
+        if (lane == 0) s_warp[threadIdx.x >> 5] = mine;
         __syncthreads();
         if (threadIdx.x == 0) {
             int t = 0;
-            for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += s_scan[w];
+#pragma unroll
+            for (int w = 0; w < kBfsThreads / 32; ++w) t += s_warp[w];
             a.block_sum[blockIdx.x] = t;
         }
         if (!bar.sync(&s_flag)) return;
         if (ld_volatile_int(a.out + 3) != 0) return;  // every block sees it: the host takes over
-        // offsets: blocks before this one, then a running scan of this block's chunk
-        if (threadIdx.x == 0) {
-            int base = 0;
-            for (int b = 0; b < static_cast<int>(blockIdx.x); ++b) base += a.block_sum[b];
-            s_run = base;
+        int run = 0, total = 0;
+        for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) {
+            const int v = a.block_sum[b];
+            total += v;
+            if (b < static_cast<int>(blockIdx.x)) run += v;
         }
-        __syncthreads();
-        int total = 0;
-        for (int b = 0; b < static_cast<int>(gridDim.x); ++b) total += a.block_sum[b];
-        for (int t0 = c0; t0 < c1; t0 += blockDim.x) {
-            const int q = t0 + threadIdx.x;
-            const int c = q < c1 ? a.cnt[q] : 0;
-            s_scan[threadIdx.x] = c;
+        run = __reduce_add_sync(0xffffffffu, run);
+        total = __reduce_add_sync(0xffffffffu, total);
+        // write
+        for (int t0 = c0; t0 < c1; t0 += kGroups) {
+            const int q = t0 + g;
+            if (!held) m = q < c1 ? a.cnt[q] : 0;
+            if (l == 0) s_cnt[g] = q < c1 ? m : 0;
             __syncthreads();
-            for (int o = 1; o < static_cast<int>(blockDim.x); o <<= 1) {
-                const int v = threadIdx.x >= static_cast<unsigned>(o) ? s_scan[threadIdx.x - o] : 0;
-                __syncthreads();
-                s_scan[threadIdx.x] += v;
-                __syncthreads();
-            }
-            const int off = s_run + s_scan[threadIdx.x] - c;
-            if (q < c1 && c > 0) {
-                const int p = lb + q, x = a.order[p];
-                int kids[kMaxChildren];
-                int m = 0;
-                for (int k = a.rp[x]; k < a.rp[x + 1]; ++k) {
-                    const int u = a.ci[k];
-                    if (u != x && a.claim[u] == p) {
-                        int j = m++;  // insertion by (degree, index)
-                        while (j > 0 && before(a.deg, u, kids[j - 1])) {
-                            kids[j] = kids[j - 1];
-                            --j;
-                        }
-                        kids[j] = u;
-                    }
-                }
+            int off = 0, tile = 0;
+            for (int i = lane; i < kGroups; i += 32) tile += s_cnt[i];
+            tile = __reduce_add_sync(0xffffffffu, tile);
+            for (int i = l; i < g; i += kLanes) off += s_cnt[i];
+            __syncwarp();
+            off = __reduce_add_sync(gmask, off) + run;
+            if (q < c1 && m > 0) {
+                if (!held) gather_children(a, a.order[lb + q], lb + q, gmask, l, kid);
                 for (int j = 0; j < m; ++j) {
-                    a.order[le + off + j] = kids[j];
-                    a.vis[kids[j]] = a.stamp;
-                    a.claim[kids[j]] = kFree;
+                    const unsigned long long key = kid[j];
+                    int rank = 0;
+                    for (int i = l; i < m; i += kLanes) rank += kid[i] < key;
+                    __syncwarp(gmask);
+                    const int pos = le + off + __reduce_add_sync(gmask, rank);
+                    const int u = static_cast<int>(key & 0xFFFFFFFFu);
+                    if (l == 0) a.order[pos] = u;
+                    const int e = a.rp[u + 1];
+                    for (int k = a.rp[u] + l; k < e; k += kLanes) {
+                        const int w = a.ci[k];
+                        if (a.claim[w] > pos) atomicMin(&a.claim[w], pos);
+                    }
+                    __syncwarp(gmask);
                 }
             }
-            __syncthreads();
-            if (threadIdx.x == 0) s_run += s_scan[blockDim.x - 1];
+            run += tile;
             __syncthreads();
         }
         if (!bar.sync(&s_flag)) return;
         lb = le;
         le += total;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.out[0] = le;
-        a.out[1] = levels;
-        a.out[2] = last_b;
-    }
+    finish_bfs(a, le, levels, last_b);
 }
 
 __global__ void k_degree(const int* __restrict__ rp, const int* __restrict__ ci, int n, int* __restrict__ deg,
@@ -193,17 +274,17 @@ __global__ void k_argmin(const int* __restrict__ order, int b, int e, const int*
     atomicMin(best, (static_cast<unsigned long long>(deg[v]) << 32) | static_cast<unsigned>(v));
 }
 
-__global__ void k_place(const int* __restrict__ order, int count, int* __restrict__ placed, int* __restrict__ result,
+__global__ void k_place(const int* __restrict__ order, int count, int* __restrict__ claim, int* __restrict__ result,
                         int pos) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= count) return;
-    placed[order[q]] = 1;
+    claim[order[q]] = -1;
     result[pos + q] = order[q];
 }
 
-__global__ void k_first_unplaced(const int* __restrict__ placed, int from, int n, int* __restrict__ first) {
+__global__ void k_first_unplaced(const int* __restrict__ claim, int from, int n, int* __restrict__ first) {
     const int i = from + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !placed[i]) atomicMin(first, i);
+    if (i < n && claim[i] == kFree) atomicMin(first, i);
 }
 
 __global__ void k_reverse(const int* __restrict__ result, int n, int* __restrict__ perm) {
@@ -244,8 +325,6 @@ struct Tmp {
 bool rcm_device(int n, const int* d_rp, const int* d_ci, int* d_perm, cudaStream_t st) {
     Tmp tmp;
     int* deg = tmp.get<int>(static_cast<size_t>(n));
-    int* placed = tmp.get<int>(static_cast<size_t>(n));
-    int* vis = tmp.get<int>(static_cast<size_t>(n));
     int* claim = tmp.get<int>(static_cast<size_t>(n));
     int* order = tmp.get<int>(static_cast<size_t>(n));
     int* result = tmp.get<int>(static_cast<size_t>(n));
@@ -255,13 +334,13 @@ bool rcm_device(int n, const int* d_rp, const int* d_ci, int* d_perm, cudaStream
     int dev = 0, sms = 0, per_sm = 0;
     ck(cudaGetDevice(&dev), "cudaGetDevice");
     ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr");
-    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs, kBfsThreads, 0), "occupancy");
-    require(per_sm > 0, XPLUS_ERR_CUDA, "rcm: the BFS kernel cannot be resident");
+    for (const auto kernel : {k_bfs, k_levels}) {
+        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBfsThreads, 0), "occupancy");
+        require(per_sm > 0, XPLUS_ERR_CUDA, "rcm: the BFS kernel cannot be resident");
+    }
     const int grid = sms;  // one block per SM, co-resident
     int* block_sum = tmp.get<int>(static_cast<size_t>(grid));
-    int* out = tmp.get<int>(4);
-    unsigned* bar = tmp.get<unsigned>(1);
-    int* err = tmp.get<int>(1);
+    int* ctl = tmp.get<int>(9);  // what a BFS starts from zeroed: out[4], tail[3], barrier counter, error flag
     const int tb = 256;
     ck(cudaMemsetAsync(small, 0, 8 * sizeof(int), st), "memset");
     k_degree<<<(n + tb - 1) / tb, tb, 0, st>>>(d_rp, d_ci, n, deg, small);
@@ -270,32 +349,24 @@ bool rcm_device(int n, const int* d_rp, const int* d_ci, int* d_perm, cudaStream
     ck(cudaMemcpyAsync(h_small, small, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
     ck(cudaStreamSynchronize(st), "sync");
     if (h_small[0]) return false;
-    ck(cudaMemsetAsync(placed, 0, static_cast<size_t>(n) * sizeof(int), st), "memset");
-    ck(cudaMemsetAsync(vis, 0, static_cast<size_t>(n) * sizeof(int), st), "memset");
     ck(cudaMemsetAsync(claim, 0x7F, static_cast<size_t>(n) * sizeof(int), st), "memset");
-    int stamp = 0;
     // one BFS from root over the unplaced nodes: {visited, levels, last level begin}
-    auto bfs = [&](int root, int (&res)[3]) -> bool {
-        ++stamp;
+    auto bfs = [&](void (*kernel)(BfsArgs), int root, int (&res)[3]) -> bool {
         BfsArgs a{};
         a.rp = d_rp;
         a.ci = d_ci;
         a.deg = deg;
-        a.placed = placed;
-        a.vis = vis;
         a.claim = claim;
         a.order = order;
         a.cnt = cnt;
         a.block_sum = block_sum;
-        a.out = out;
-        a.stamp = stamp;
+        a.out = ctl;
+        a.tail = ctl + 4;
         a.root = root;
-        a.bar = bar;
-        a.err = err;
+        a.bar = reinterpret_cast<unsigned*>(ctl + 7);
+        a.err = ctl + 8;
         a.timeout_ns = 2000000000LL;
-        ck(cudaMemsetAsync(out, 0, 4 * sizeof(int), st), "memset");
-        ck(cudaMemsetAsync(bar, 0, sizeof(unsigned), st), "memset");
-        ck(cudaMemsetAsync(err, 0, sizeof(int), st), "memset");
+        ck(cudaMemsetAsync(ctl, 0, 9 * sizeof(int), st), "memset");
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
         cfg.blockDim = dim3(kBfsThreads);
@@ -305,12 +376,11 @@ bool rcm_device(int n, const int* d_rp, const int* d_ci, int* d_perm, cudaStream
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        ck(cudaLaunchKernelEx(&cfg, k_bfs, a), "rcm BFS launch");
-        int h_out[4], h_err = 0;
-        ck(cudaMemcpyAsync(h_out, out, sizeof(h_out), cudaMemcpyDeviceToHost, st), "D2H");
-        ck(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
+        ck(cudaLaunchKernelEx(&cfg, kernel, a), "rcm BFS launch");
+        int h_out[9];
+        ck(cudaMemcpyAsync(h_out, ctl, sizeof(h_out), cudaMemcpyDeviceToHost, st), "D2H");
         ck(cudaStreamSynchronize(st), "sync");
-        require(h_err == 0, XPLUS_ERR_CUDA, "rcm: a grid barrier timed out");
+        require(h_out[8] == 0, XPLUS_ERR_CUDA, "rcm: a grid barrier timed out");
         if (h_out[3]) return false;
         res[0] = h_out[0];
         res[1] = h_out[1];
@@ -332,19 +402,19 @@ bool rcm_device(int n, const int* d_rp, const int* d_ci, int* d_perm, cudaStream
         // the lowest unplaced node
         const int big = INT_MAX;
         ck(cudaMemcpyAsync(small + 1, &big, sizeof(int), cudaMemcpyHostToDevice, st), "H2D");
-        k_first_unplaced<<<(n - seed + tb - 1) / tb, tb, 0, st>>>(placed, seed, n, small + 1);
+        k_first_unplaced<<<(n - seed + tb - 1) / tb, tb, 0, st>>>(claim, seed, n, small + 1);
         ck(cudaGetLastError(), "rcm seed");
         ck(cudaMemcpyAsync(&seed, small + 1, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
         ck(cudaStreamSynchronize(st), "sync");
         int r[3];
-        if (!bfs(seed, r)) return false;
+        if (!bfs(k_levels, seed, r)) return false;
         int v = argmin(0, r[0]);  // the component's minimum-(degree, index) node
-        if (!bfs(v, r)) return false;
+        if (!bfs(k_levels, v, r)) return false;
         int ecc = r[1], last_b = r[2], last_e = r[0];
         while (true) {  // George-Liu pseudo-peripheral node
             const int u = argmin(last_b, last_e);
             int r2[3];
-            if (!bfs(u, r2)) return false;
+            if (!bfs(k_levels, u, r2)) return false;
             if (r2[1] > ecc) {
                 v = u;
                 ecc = r2[1];
@@ -354,8 +424,8 @@ bool rcm_device(int n, const int* d_rp, const int* d_ci, int* d_perm, cudaStream
                 break;
             }
         }
-        if (!bfs(v, r)) return false;  // Cuthill-McKee from v
-        k_place<<<(r[0] + tb - 1) / tb, tb, 0, st>>>(order, r[0], placed, result, pos);
+        if (!bfs(k_bfs, v, r)) return false;  // Cuthill-McKee from v
+        k_place<<<(r[0] + tb - 1) / tb, tb, 0, st>>>(order, r[0], claim, result, pos);
         ck(cudaGetLastError(), "rcm place");
         pos += r[0];
     }
