@@ -504,7 +504,7 @@ int xplus_gen_fem3d(int g, double sigma, double jitter, uint64_t seed, int64_t p
 /* Reverse Cuthill-McKee ordering of a structurally symmetric CSR: perm[new] = old. */
 int xplus_rcm(int n, const int* row_ptr, const int* col_idx, int* perm);
 /* The same reverse Cuthill-McKee ordering computed on the GPU from a device CSR, bit-identical
- * to xplus_rcm: one cooperative launch per BFS builds the Cuthill-McKee levels in parallel
+ * to xplus_rcm: one cooperative launch builds the Cuthill-McKee levels in parallel
  * (each node of the next level goes to its lowest-positioned neighbour in the current level,
  * each parent's children ordered by (degree, index)), the pseudo-peripheral search and the
  * component order as xplus_rcm has them.  A graph it does not cover (a node with more than 64
