@@ -778,6 +778,8 @@ __global__ void __launch_bounds__(512, 1) pcg_resident1_kernel(PcgArgs a) {
                 }
             }
             __syncthreads();
+            // the update is applied: a breakdown at p'.Ap' or alpha leaves none to apply at the exit
+            if (threadIdx.x == 0) st.pend = 0.0;
             clock(2);
             // ---- Ap' from shared memory, then each row's records of the next generation and
             // its terms of the seven sums (the row's own values only: no CTA barrier between) ----
