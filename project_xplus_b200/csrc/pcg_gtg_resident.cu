@@ -71,7 +71,7 @@ __device__ __forceinline__ void g_rows(const GSlots& m, const float* x, int w0, 
             const int2 sl = m.table[s - m.sb];
             const bool staged = s < m.sm_end;
             const int off = sl.x - (staged ? m.m0 : 0) + lane * 2;
-            w[k] = sl.y;  // at least 2: every row has its diagonal
+            w[k] = sl.y;  // at least 2: a G or G^T with a slice without slots does not come here
             wmax = max(wmax, sl.y);
             vp[k] = (staged ? m.mval : m.val) + off;
             cp[k] = (staged ? m.mcol : m.col) + off;
@@ -655,7 +655,7 @@ GtgKernel pick(const KernelKey& k) {
     return nullptr;
 }
 
-// thread per SELL row of a chunk-2 image
+// thread per SELL row of a chunk-2 image whose rows' columns lie within 32767 of them
 __global__ void k_gtg_pack16(const long long* __restrict__ slice_ptr, int n_pad, const int* __restrict__ col,
                              short* __restrict__ col16) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
@@ -669,9 +669,11 @@ __global__ void k_gtg_pack16(const long long* __restrict__ slice_ptr, int n_pad,
     }
 }
 
-__global__ void __launch_bounds__(256) k_gtg_windows(const long long* __restrict__ slice_ptr,
-                                                     const short* __restrict__ col16, int chunk, int n_slices, int n_pad,
-                                                     int per, int2* __restrict__ win) {
+// The window of band blockIdx.x over the columns of A (offsets from the row), G and G^T.  The three
+// patterns differ where A stores one of (i, j) and (j, i) alone: G^T's row j then reaches a column
+// that A's row j does not have.  *empty: some slice of G or G^T has no slots.
+__global__ void __launch_bounds__(256) k_gtg_windows(GtgPatterns m, int n_slices, int n_pad, int per,
+                                                     int2* __restrict__ win, int* __restrict__ empty) {
     __shared__ int s_lo, s_hi;
     const int sb = blockIdx.x * per, se = min(n_slices, sb + per);
     if (threadIdx.x == 0) {
@@ -681,12 +683,23 @@ __global__ void __launch_bounds__(256) k_gtg_windows(const long long* __restrict
     __syncthreads();
     int lo = sb * 32, hi = se * 32;
     for (int s = sb + static_cast<int>(threadIdx.x >> 5); s < se; s += 8) {
-        const long long b0 = slice_ptr[s];
-        const int slots = static_cast<int>(slice_ptr[s + 1] - b0);
+        const long long b0 = m.slice_ptr[s];
+        const int slots = static_cast<int>(m.slice_ptr[s + 1] - b0);
         for (int q = threadIdx.x & 31; q < slots; q += 32) {
-            const int c = s * 32 + (q / chunk) % 32 + col16[b0 + q];
+            const int c = s * 32 + (q / m.chunk) % 32 + m.col16[b0 + q];
             lo = min(lo, c);
             hi = max(hi, c + 1);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const long long* __restrict__ sp = k == 0 ? m.g_slice_ptr : m.gt_slice_ptr;
+            const int* __restrict__ col = k == 0 ? m.g_col : m.gt_col;
+            const long long e = sp[s + 1];
+            if (sp[s] == e) *empty = 1;
+            for (long long q = sp[s] + (threadIdx.x & 31); q < e; q += 32) {
+                lo = min(lo, col[q]);
+                hi = max(hi, col[q] + 1);
+            }
         }
     }
     atomicMin(&s_lo, lo);
@@ -752,9 +765,8 @@ cudaError_t gtg_pack16(const long long* slice_ptr, int n_slices, const int* col,
     return cudaGetLastError();
 }
 
-cudaError_t gtg_windows(const long long* slice_ptr, const short* col16, int chunk, int n_slices, int n_pad, int grid,
-                        int2* win, cudaStream_t s) {
-    k_gtg_windows<<<grid, 256, 0, s>>>(slice_ptr, col16, chunk, n_slices, n_pad, (n_slices + grid - 1) / grid, win);
+cudaError_t gtg_windows(const GtgPatterns& m, int n_slices, int n_pad, int grid, int2* win, int* empty, cudaStream_t s) {
+    k_gtg_windows<<<grid, 256, 0, s>>>(m, n_slices, n_pad, (n_slices + grid - 1) / grid, win, empty);
     return cudaGetLastError();
 }
 

@@ -128,11 +128,16 @@ size_t gtg_res_vector_bytes(int rows, int window);
 cudaError_t gtg_res_prepare(const KernelKey& k, int device, size_t vector_bytes, size_t matrix_bytes, bool* fits,
                             size_t* smem_bytes);
 cudaError_t gtg_res_launch(const KernelKey& k, const PcgArgs& a, int grid, size_t smem_bytes, cudaStream_t s);
-// int16 offsets of a G or G^T image (chunk 2, |col - row| < 32768), and per block of `grid` the window
-// {first row, rows} that the columns of A (int16 offsets) reach, widened to multiples of 4
+// int16 offsets of a G or G^T image (chunk 2, |col - row| < 32768)
 cudaError_t gtg_pack16(const long long* slice_ptr, int n_slices, const int* col, short* col16, cudaStream_t s);
-cudaError_t gtg_windows(const long long* slice_ptr, const short* col16, int chunk, int n_slices, int n_pad, int grid,
-                        int2* win, cudaStream_t s);
+// Per block of `grid` the window {first row, rows}, widened to multiples of 4, that the columns of A
+// (int16 offsets), G and G^T (int32 columns) reach; *empty becomes 1 when a slice of G or G^T has no slots.
+struct GtgPatterns {
+    const long long* slice_ptr; const short* col16; int chunk;
+    const long long *g_slice_ptr, *gt_slice_ptr;
+    const int *g_col, *gt_col;
+};
+cudaError_t gtg_windows(const GtgPatterns& m, int n_slices, int n_pad, int grid, int2* win, int* empty, cudaStream_t s);
 // val[q] = glow[map[q]] (0 where map[q] < 0): G values into a SELL image of G or G^T
 cudaError_t gtg_fill_values(const double* d_glow, const int* d_map, float* d_val, long long slots, cudaStream_t s);
 cudaError_t spmv_launch(const KernelKey& k, const SpmvArgs& a, const void* x, void* y,

@@ -874,17 +874,25 @@ void gtg_layout_host(xplus_pcg* h, const int* row_ptr, const int* col_idx) {
     cuda_check(cudaStreamSynchronize(st), "sync");  // the host images go next
 }
 
-// The SM-resident G^T G kernel, when the handle's bands fit it: windows, int16 offsets of G and G^T
-// (their patterns lie within A's, whose offsets are int16), shared memory.
+// The SM-resident G^T G kernel, when the handle's bands fit it: windows, int16 offsets of G and G^T,
+// shared memory.  Windows and offsets come from the images themselves, whatever pattern they have:
+// with A's alone a one-sided entry of A, or a pattern given to xplus_pcg_set_gtg that is not A's,
+// would make the kernel gather outside its shared memory.
 void gtg_resident(xplus_pcg* h) {
     const int grid = h->gtg_grid, per = (h->n_slices + grid - 1) / grid;
     if (!gtg_res_supported(h->key) || !h->opts.resident || per > kGtgResSlices) return;
     cudaStream_t st = h->stream;
+    CreateTmp tmp;
+    int* d_empty = tmp.get<int>(1);
+    cuda_check(cudaMemsetAsync(d_empty, 0, sizeof(int), st), "memset");
     h->d_gtg_win = dalloc<int2>(h, static_cast<size_t>(grid));
-    cuda_check(gtg_windows(h->d_slice_ptr, static_cast<const short*>(h->d_col), h->opts.chunk, h->n_slices, h->n_pad, grid,
-                           h->d_gtg_win, st), "gtg windows");
+    const GtgPatterns pattern{h->d_slice_ptr, static_cast<const short*>(h->d_col), h->opts.chunk, h->d_g_slice_ptr,
+                              h->d_gt_slice_ptr, h->d_g_col, h->d_gt_col};
+    cuda_check(gtg_windows(pattern, h->n_slices, h->n_pad, grid, h->d_gtg_win, d_empty, st), "gtg windows");
     const int bands = (h->n_slices + per - 1) / per;
+    int empty = 0;
     std::vector<int2> win(static_cast<size_t>(grid));
+    cuda_check(cudaMemcpyAsync(&empty, d_empty, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
     cuda_check(cudaMemcpyAsync(win.data(), h->d_gtg_win, win.size() * sizeof(int2), cudaMemcpyDeviceToHost, st), "D2H");
     // first slots of the bands in A, G and G^T
     const long long* sp[3] = {h->d_slice_ptr, h->d_g_slice_ptr, h->d_gt_slice_ptr};
@@ -897,6 +905,9 @@ void gtg_resident(xplus_pcg* h) {
         bp[m][static_cast<size_t>(bands)] = total[m];
     }
     cuda_check(cudaStreamSynchronize(st), "sync");
+    if (empty) return;  // the kernel's rows of G and G^T have a first pair of slots
+    for (const int2& w : win)
+        if (w.y > 32768) return;  // its offsets are int16 (12 bytes a row: such a window would not fit either)
     size_t vec = 0;
     long long mat = 0;
     for (int b = 0; b < bands; ++b) {
