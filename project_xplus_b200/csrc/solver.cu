@@ -89,6 +89,7 @@ struct xplus_pcg {
     int *d_g_col = nullptr, *d_gt_col = nullptr, *d_g_map = nullptr, *d_gt_map = nullptr;
     float *d_g_val = nullptr, *d_gt_val = nullptr, *d_t = nullptr, *d_r2 = nullptr;
     double* d_glow = nullptr;
+    bool gtg_ready = false;    // the images and vectors below are complete
     bool gtg_res = false;      // its SM-resident form (pcg_gtg_resident.cu)
     size_t gtg_smem = 0;
     short *d_g_col16 = nullptr, *d_gt_col16 = nullptr;
@@ -916,21 +917,24 @@ void gtg_resident(xplus_pcg* h) {
         mat = std::max(mat, (bp[0][k + 1] - bp[0][k]) * static_cast<long long>(elem_size(h->opts.value_type) + 2) +
                                 (bp[1][k + 1] - bp[1][k] + bp[2][k + 1] - bp[2][k]) * 6);
     }
-    cuda_check(gtg_res_prepare(h->key, h->device, vec, static_cast<size_t>(mat), &h->gtg_res, &h->gtg_smem), "gtg resident");
-    if (!h->gtg_res) return;
+    bool fits = false;
+    cuda_check(gtg_res_prepare(h->key, h->device, vec, static_cast<size_t>(mat), &fits, &h->gtg_smem), "gtg resident");
+    if (!fits) return;
     h->d_g_col16 = dalloc<short>(h, static_cast<size_t>(h->g_slots));
     h->d_gt_col16 = dalloc<short>(h, static_cast<size_t>(h->gt_slots));
     cuda_check(gtg_pack16(h->d_g_slice_ptr, h->n_slices, h->d_g_col, h->d_g_col16, st), "gtg pack");
     cuda_check(gtg_pack16(h->d_gt_slice_ptr, h->n_slices, h->d_gt_col, h->d_gt_col16, st), "gtg pack");
+    h->gtg_res = true;
 }
 
 // The G / G^T images and the vectors of the G^T G kernel for the pattern of the CSR given to
-// xplus_pcg_create (once per handle): on the GPU unless the handle was built on the host.
+// xplus_pcg_create (once per handle, and again after a call that failed halfway): on the GPU unless
+// the handle was built on the host.
 void gtg_layout(xplus_pcg* h, const int* row_ptr, const int* col_idx) {
     require(h->opts.vector_type == XPLUS_F32 && h->key.diag && h->opts.value_type != XPLUS_F64,
             XPLUS_ERR_ARG, "G^T G preconditioning needs FP32 vectors, FP32, BF16 or FP16 values and row_sum_form");
     require(h->d_val64 != nullptr, XPLUS_ERR_ARG, "G^T G preconditioning needs keep_fp64");
-    if (h->d_g_slice_ptr) return;
+    if (h->gtg_ready) return;
     const int n = h->n;
     require(row_ptr && col_idx && row_ptr[0] == 0 && row_ptr[n] == h->nnz, XPLUS_ERR_ARG,
             "pattern differs from the matrix of the handle");
@@ -965,8 +969,13 @@ void gtg_layout(xplus_pcg* h, const int* row_ptr, const int* col_idx) {
         h->d_partial = dalloc<double>(h, static_cast<size_t>(16) * h->gtg_grid);
         h->d_block_clk = dalloc<long long>(h, static_cast<size_t>(4) * h->gtg_grid);
     }
-    gtg_resident(h);
+    try {
+        gtg_resident(h);
+    } catch (const Error& e) {
+        if (e.code != XPLUS_ERR_NOMEM) throw;  // no room for its arrays: the global-memory form does without
+    }
     cuda_check(cudaStreamSynchronize(st), "sync");
+    h->gtg_ready = true;
 }
 
 // G values (device, g_low order) -> the two SELL images; switches the handle to G^T G
