@@ -719,8 +719,8 @@ size_t gtg_res_vector_bytes(int rows, int window) {
     return 20 * static_cast<size_t>(rows) + 12 * static_cast<size_t>(window);
 }
 
-cudaError_t gtg_res_prepare(const KernelKey& k, int device, size_t vector_bytes, size_t matrix_bytes, bool* fits,
-                            size_t* smem_bytes) {
+cudaError_t gtg_res_prepare(const KernelKey& k, int device, int grid, size_t vector_bytes, size_t matrix_bytes,
+                            bool* fits, size_t* smem_bytes) {
     *fits = false;
     GtgKernel f = pick(k);
     if (!f) return cudaSuccess;
@@ -736,11 +736,13 @@ cudaError_t gtg_res_prepare(const KernelKey& k, int device, size_t vector_bytes,
     e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit));
     if (e != cudaSuccess) return e;
     const size_t want = std::min(limit, vector_bytes + matrix_bytes);
-    int per_sm = 0;
+    int per_sm = 0, sms = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 512, want);
     if (e != cudaSuccess) return e;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return e;
     *smem_bytes = want;
-    *fits = per_sm >= 1;
+    *fits = grid <= per_sm * sms;  // the grid is the global-memory kernel's, all of it must be resident
     return cudaSuccess;
 }
 

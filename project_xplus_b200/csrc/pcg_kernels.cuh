@@ -125,8 +125,8 @@ cudaError_t gtg_launch(const KernelKey& k, const PcgArgs& a, int grid, int tpb, 
 constexpr int kGtgResSlices = 256;  // slice table capacity per CTA
 bool gtg_res_supported(const KernelKey& k);
 size_t gtg_res_vector_bytes(int rows, int window);
-cudaError_t gtg_res_prepare(const KernelKey& k, int device, size_t vector_bytes, size_t matrix_bytes, bool* fits,
-                            size_t* smem_bytes);
+cudaError_t gtg_res_prepare(const KernelKey& k, int device, int grid, size_t vector_bytes, size_t matrix_bytes,
+                            bool* fits, size_t* smem_bytes);
 cudaError_t gtg_res_launch(const KernelKey& k, const PcgArgs& a, int grid, size_t smem_bytes, cudaStream_t s);
 // int16 offsets of a G or G^T image (chunk 2, |col - row| < 32768)
 cudaError_t gtg_pack16(const long long* slice_ptr, int n_slices, const int* col, short* col16, cudaStream_t s);

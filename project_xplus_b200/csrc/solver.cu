@@ -918,7 +918,7 @@ void gtg_resident(xplus_pcg* h) {
                                 (bp[1][k + 1] - bp[1][k] + bp[2][k + 1] - bp[2][k]) * 6);
     }
     bool fits = false;
-    cuda_check(gtg_res_prepare(h->key, h->device, vec, static_cast<size_t>(mat), &fits, &h->gtg_smem), "gtg resident");
+    cuda_check(gtg_res_prepare(h->key, h->device, grid, vec, static_cast<size_t>(mat), &fits, &h->gtg_smem), "gtg resident");
     if (!fits) return;
     h->d_g_col16 = dalloc<short>(h, static_cast<size_t>(h->g_slots));
     h->d_gt_col16 = dalloc<short>(h, static_cast<size_t>(h->gt_slots));
