@@ -91,10 +91,14 @@ typedef struct xplus_opts {
                               matrix and multiplies the iteration count */
     int index16;           /* store columns as int16 offsets from the row when every |col - row|
                               < 32768 after ordering (lossless; default 1) */
-    int l2_persist;        /* mark the matrix stream as persisting in L2 for the solve launch
-                              (default 1).  Raises this process's persisting-L2 limit while the
-                              handle exists; destroying the handle releases its persisting lines
-                              and the last such handle restores the previous limit */
+    int l2_persist;        /* mark the matrix stream as persisting in L2 for the solve launches of
+                              the global-memory kernels, Jacobi and G^T G (default 1; the other
+                              kernels ask for no part of L2).  Raises this process's persisting-L2
+                              limit while the handle uses such a kernel; destroying it, or going
+                              back to Jacobi on another kernel, releases its persisting lines, and
+                              the last such handle restores the previous limit.  The limit is the
+                              device's: a windowed solve beside such a handle is slower (128^3:
+                              50 us per iteration alone, 74 beside one) */
     int resident;          /* FP32 vectors, row-sum form: use the SM-resident kernel (state and
                               the search direction's band + halo in shared memory) when one CTA
                               per SM holds it (default 1) */

@@ -251,19 +251,24 @@ std::mutex g_l2_mutex;
 std::multiset<size_t> g_l2_wants;
 size_t g_l2_limit_before = 0;
 
+// Hands the handle's share of L2 back (after its solves: the matrix's lines stay persisting until reset).
+void release_l2(xplus_pcg* h) {
+    if (!h->l2_user) return;
+    cudaCtxResetPersistingL2Cache();
+    std::lock_guard<std::mutex> lk(g_l2_mutex);
+    const auto it = g_l2_wants.find(h->l2_want);
+    if (it != g_l2_wants.end()) g_l2_wants.erase(it);
+    const size_t keep = g_l2_wants.empty() ? g_l2_limit_before : std::max(g_l2_limit_before, *g_l2_wants.rbegin());
+    cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, keep);
+    h->l2_user = false;
+    h->window = cudaAccessPolicyWindow{};
+}
+
 void destroy(xplus_pcg* h) {
     if (!h) return;
     if (h->device >= 0) cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    if (h->l2_user) {
-        // the matrix's lines stay persisting in L2 until reset: hand the cache back
-        cudaCtxResetPersistingL2Cache();
-        std::lock_guard<std::mutex> lk(g_l2_mutex);
-        const auto it = g_l2_wants.find(h->l2_want);
-        if (it != g_l2_wants.end()) g_l2_wants.erase(it);
-        const size_t keep = g_l2_wants.empty() ? g_l2_limit_before : std::max(g_l2_limit_before, *g_l2_wants.rbegin());
-        cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, keep);
-    }
+    release_l2(h);
     for (void* p : h->allocations) cudaFree(p);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
@@ -1239,7 +1244,10 @@ int xplus_pcg_set_gtg(xplus_pcg* h, const int* row_ptr, const int* col_idx, cons
         require(h, XPLUS_ERR_ARG, "null handle");
         cuda_check(cudaSetDevice(h->device), "cudaSetDevice");
         if (!g_low) {
+            // back to Jacobi: only the global-memory kernel wants a part of L2 set aside (the windowed
+            // kernel loses by it: 128^3, 50.4 us per iteration without, 73.5 with)
             h->gtg = false;
+            if (h->resident || h->windowed || h->small) release_l2(h);
             return;
         }
         require(fallback_iters >= 0, XPLUS_ERR_ARG, "fallback_iters must be >= 0");
