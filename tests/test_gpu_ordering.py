@@ -58,3 +58,11 @@ def test_components_and_single_nodes(gpu):
     """Paths, cycles and nodes without neighbours, relabelled together."""
     edges = [(i, i + 1) for i in range(40)] + [(50 + i, 50 + (i + 1) % 17) for i in range(17)] + [(80, 81)]
     _same(*_csr(100, edges, seed=3))
+
+
+@pytest.mark.parametrize("leaves", [64, 65, 200])
+def test_a_wide_root_is_seen_in_the_first_search(gpu, leaves):
+    """Node 0, where the first search starts, has a path of ten nodes and the leaves: as many children as neighbours there,
+    one fewer in the order from the far end.  The host takes over as soon as a search counts more than 64."""
+    path = [(i, i + 1) for i in range(9)]
+    _same(*_csr(10 + leaves, path + [(0, 10 + k) for k in range(leaves - 1)]), on_gpu=leaves <= 64)
