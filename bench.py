@@ -446,7 +446,7 @@ def run_b200(args):
             r3 = runs[-1]
             mixed_3d[name] = {"time_to_tol_ms": r3.kernel_ms, "iterations": r3.iterations, "status": r3.status,
                               "replacements": r3.replacements, "true_rel_residual": r3.residual_rel,
-                              "stagnated": r3.metrics["stagnated"], "kernel": r3.metrics["kernel"],
+                              "stagnated": r3.metrics["stagnated"], "kernel": r3.metrics["kernel_form"],
                               "slots": s3.info()["slots"]}
             s3.close()
         if rank == 0 and world == 1 and not args.no_cpu_baseline:

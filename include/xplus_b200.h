@@ -139,18 +139,30 @@ typedef struct xplus_opts {
                               diverges), FP16 836 in 91 ms, FP32 values 807 in 90 ms */
 } xplus_opts;
 
+/* ---- xplus_metrics.kernel ---- */
+#define XPLUS_KERNEL_PERSISTENT 1 /* pcg_persistent_kernel: state in global memory */
+#define XPLUS_KERNEL_SMALL 2      /* pcg_small_kernel: one CTA, FP64 vectors */
+#define XPLUS_KERNEL_WINDOW 3     /* pcg_window_kernel: the search direction's window in shared memory */
+#define XPLUS_KERNEL_RESIDENT 4   /* pcg_resident_kernel: SM-resident, two barriers per iteration */
+#define XPLUS_KERNEL_RESIDENT1 5  /* pcg_resident1_kernel: SM-resident, one barrier */
+#define XPLUS_KERNEL_GTG 6        /* pcg_gtg_kernel: G^T G, state in global memory */
+#define XPLUS_KERNEL_GTG_RES 7    /* pcg_gtg_res_kernel: G^T G, SM-resident */
+
 typedef struct xplus_metrics {
     int status;            /* XPLUS_CONVERGED .. XPLUS_TIMEOUT */
     int iterations;        /* inner PCG iterations (status[1] of the control kernel) */
     int replacements;      /* FP64 residual replacements performed */
-    int reserved0;
+    int kernel;            /* kernel of the last solve launch, XPLUS_KERNEL_* (0: none yet) */
     double rz, rr, pap, alpha;  /* metrics[0..3] of the control kernel */
     double true_rel_residual;   /* FP64 ||b - A x|| / ||b|| at exit (when the FP64 copy exists) */
     double kernel_ms;           /* device time of the solve launch(es) */
     double setup_ms;            /* host+device time of xplus_pcg_create */
     double reserved[4];         /* [0] stagnation stop (1/0), [1] device time from the kernel's
-                                   own clock (ms), [2] kernel: 0 global-memory persistent,
-                                   1 SM-resident two-barrier, 2 SM-resident one-barrier */
+                                   own clock (ms), [2] iteration scheme: 0 two reductions, state in
+                                   global memory or of one CTA, 1 SM-resident two-barrier,
+                                   2 SM-resident one-barrier, 3 G^T G (its forms, and those of 0,
+                                   are one arithmetic: `kernel` tells them apart), [3] with 3 the
+                                   iteration of the switch to Jacobi (-1: none) */
 } xplus_metrics;
 
 typedef struct xplus_pcg xplus_pcg;      /* one SPD system resident on one GPU */

@@ -38,7 +38,7 @@ class XplusOpts(C.Structure):
 class XplusMetrics(C.Structure):
     _fields_ = [
         ("status", C.c_int), ("iterations", C.c_int), ("replacements", C.c_int),
-        ("reserved0", C.c_int), ("rz", C.c_double), ("rr", C.c_double), ("pap", C.c_double),
+        ("kernel", C.c_int), ("rz", C.c_double), ("rr", C.c_double), ("pap", C.c_double),
         ("alpha", C.c_double), ("true_rel_residual", C.c_double), ("kernel_ms", C.c_double),
         ("setup_ms", C.c_double), ("reserved", C.c_double * 4),
     ]

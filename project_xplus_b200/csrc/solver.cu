@@ -72,6 +72,7 @@ struct xplus_pcg {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     xplus_metrics last{};
     bool pending = false;
+    int launched = 0;          // XPLUS_KERNEL_* of the last solve
     int debug_skip_block = -1;
     long long phase_ns[4] = {0, 0, 0, 0};
     std::vector<void*> allocations;
@@ -753,21 +754,29 @@ void enqueue_solve(xplus_pcg* h, double tau, int tau_mode, int max_iters_in, int
             a.smem_bytes = static_cast<int>(h->gtg_smem);
             a.z = h->d_rec;
             cuda_check(gtg_res_launch(h->key, a, h->gtg_grid, h->gtg_smem, st), "resident GTG PCG launch");
-        } else
+            h->launched = XPLUS_KERNEL_GTG_RES;
+        } else {
             cuda_check(gtg_launch(h->key, a, h->gtg_grid, 512, st, h->window), "GTG PCG launch");
-    } else if (h->resident)
+            h->launched = XPLUS_KERNEL_GTG;
+        }
+    } else if (h->resident) {
         // no access-policy window: the resident kernel's only global stream is a matrix that L2
         // holds anyway, and the launch attribute cost time (1108^2 system: 97.1 ms with it,
         // 95.9 ms without, and ~3 ms more on the host per solve call)
         cuda_check(resident_launch(h->key, a, h->grid, h->tpb, h->smem_bytes, h->one_sync, st,
                                    cudaAccessPolicyWindow{}),
                    "resident PCG launch");
-    else if (h->windowed)
+        h->launched = h->one_sync ? XPLUS_KERNEL_RESIDENT1 : XPLUS_KERNEL_RESIDENT;
+    } else if (h->windowed) {
         cuda_check(window_launch(h->key, a, h->grid, h->tpb, h->smem_bytes, st), "windowed PCG launch");
-    else if (h->small && h->debug_skip_block < 0)
+        h->launched = XPLUS_KERNEL_WINDOW;
+    } else if (h->small && h->debug_skip_block < 0) {
         cuda_check(small_launch(h->key, a, h->tpb, h->smem_bytes, st), "one-CTA PCG launch");
-    else
+        h->launched = XPLUS_KERNEL_SMALL;
+    } else {
         cuda_check(pcg_launch(h->key, a, h->grid, h->tpb, st, h->window), "persistent PCG launch");
+        h->launched = XPLUS_KERNEL_PERSISTENT;
+    }
     cuda_check(cudaEventRecord(h->ev1, st), "event");
     h->pending = true;
 }
@@ -795,8 +804,10 @@ void collect(xplus_pcg* h, xplus_metrics* m) {
         L.kernel_ms = ms;
         L.reserved[0] = o.stagnated;
         L.reserved[1] = static_cast<double>(o.t_end_ns - o.t_start_ns) * 1e-6;
-        L.reserved[2] = h->gtg ? 3.0 : (h->resident ? (h->one_sync ? 2.0 : 1.0) : 0.0);
-        L.reserved[3] = h->gtg ? o.reserved : -1.0;
+        L.kernel = h->launched;
+        const bool gtg = h->launched == XPLUS_KERNEL_GTG || h->launched == XPLUS_KERNEL_GTG_RES;
+        L.reserved[2] = gtg ? 3.0 : (h->launched == XPLUS_KERNEL_RESIDENT1 ? 2.0 : (h->launched == XPLUS_KERNEL_RESIDENT ? 1.0 : 0.0));
+        L.reserved[3] = gtg ? o.reserved : -1.0;
         h->phase_ns[0] = o.t_phase[0];
         h->phase_ns[1] = o.t_phase[1];
         h->phase_ns[2] = o.t_phase[2];

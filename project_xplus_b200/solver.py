@@ -37,8 +37,12 @@ class run_defaults:  # noqa: N801  (mirrors the reference namespace)
 
 
 kBreakdownEps = 1.0e-30
+# iteration schemes (metrics["kernel"]), named by the kernel that defines each one's arithmetic
 KERNEL_NAMES = {0: "pcg_persistent_kernel", 1: "pcg_resident_kernel", 2: "pcg_resident1_kernel",
                 3: "pcg_gtg_kernel"}
+# kernels (metrics["kernel_form"]): what the last solve launched
+KERNEL_FORMS = {0: "none", 1: "pcg_persistent_kernel", 2: "pcg_small_kernel", 3: "pcg_window_kernel",
+                4: "pcg_resident_kernel", 5: "pcg_resident1_kernel", 6: "pcg_gtg_kernel", 7: "pcg_gtg_res_kernel"}
 kMaxN = 1024  # the reference multi-kernel cap; the GPU path has none
 
 
@@ -163,6 +167,7 @@ def _type(t) -> int:
 def _metrics_dict(m) -> dict:
     return dict(rz=m.rz, rr=m.rr, pap=m.pap, alpha=m.alpha, stagnated=bool(m.reserved[0]),
                 device_ms=m.reserved[1], kernel=KERNEL_NAMES.get(int(m.reserved[2]), "unknown"),
+                kernel_form=KERNEL_FORMS.get(m.kernel, "unknown"),
                 jacobi_fallback_at=int(m.reserved[3]) if int(m.reserved[2]) == 3 else -1)
 
 

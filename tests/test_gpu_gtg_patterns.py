@@ -38,6 +38,7 @@ def _same(matrix, b, pattern, g, tau=1e-8, tau_mode=xp.XPLUS_TAU_REL_TRUE, max_i
         out.append(s.solve(b, np.linspace(-1, 1, len(b)), tau=tau, tau_mode=tau_mode, max_iters=max_iters, trace=True))
         s.close()
     a, c = out
+    assert c.metrics["kernel_form"] == "pcg_gtg_kernel"
     assert (a.status, a.iterations, a.replacements) == (c.status, c.iterations, c.replacements)
     np.testing.assert_array_equal(a.solution, c.solution)
     np.testing.assert_array_equal([t.rr for t in a.iteration_trace], [t.rr for t in c.iteration_trace])
@@ -54,6 +55,9 @@ def test_one_sided_zeros(side, reach, lower, kw):
     exact = fsai_lower(*m)
     r = _same(m, d.b, m, exact, max_iters=2000, **kw)
     assert r.status == "converged" or kw.get("values_dtype") == "bf16"
+    # 12 bytes of shared memory per row of a window: all 91^2 rows fit, 30000 do not
+    if side < 274 or reach == 30000:
+        assert r.metrics["kernel_form"] == ("pcg_gtg_res_kernel" if side < 274 else "pcg_gtg_kernel")
     # and with values at the one-sided entries too
     _same(m, d.b, m, np.where(exact == 0.0, 0.01, exact), **kw)
 
@@ -61,7 +65,8 @@ def test_one_sided_zeros(side, reach, lower, kw):
 def test_an_offset_that_fits_int16_on_one_side_only():
     d = gen.fem2d(190, sigma=1.0, seed=2)[0]
     m = _with_zeros(d, np.array([32768, 33000]), np.array([0, 232]))  # -32768 in G, +32768 in G^T
-    _same(m, d.b, m, np.where(fsai_lower(*m) == 0.0, 0.01, fsai_lower(*m)), sigma=1)
+    r = _same(m, d.b, m, np.where(fsai_lower(*m) == 0.0, 0.01, fsai_lower(*m)), sigma=1)
+    assert r.metrics["kernel_form"] == "pcg_gtg_kernel"
 
 
 @pytest.mark.parametrize("side", [23, 91, 274])
@@ -82,5 +87,6 @@ def test_a_slice_of_g_without_entries(first):
     k = np.arange(d.nnz) - d.row_ptr[rows]
     above = (rows >= first) & (rows < first + 32) & (rows < d.n - 10)
     ci = np.where(above, rows + 1 + k, d.col_idx).astype(np.int32)
-    _same((d.row_ptr, d.col_idx, d.values), d.b, (d.row_ptr, ci), _g(d.row_ptr, ci), tau=1e-20,
-          tau_mode=xp.XPLUS_TAU_ABS_RR, max_iters=30, sigma=1)
+    r = _same((d.row_ptr, d.col_idx, d.values), d.b, (d.row_ptr, ci), _g(d.row_ptr, ci), tau=1e-20,
+              tau_mode=xp.XPLUS_TAU_ABS_RR, max_iters=30, sigma=1)
+    assert r.metrics["kernel_form"] == "pcg_gtg_kernel"
