@@ -419,7 +419,7 @@ __device__ __forceinline__ int thread_index() {
     return t;
 }
 
-// STREAM: the slots (none of them in shared memory) are read past L1 and are the first to leave L2.
+// STREAM: the slots (none of them in shared memory) are read past L1.
 template <typename VT, int CHUNK, int DEPTH, bool STREAM = false>
 struct SlotRing {
     using RV = typename RawVec<typename RawOf<VT>::type, CHUNK>::type;

@@ -11,13 +11,13 @@
 // The global-memory form gathers {z, p} records through L1 behind each slot load: two dependent
 // round trips for 16 warps, and 8 bytes per row where 4 are enough.
 //
-// The matrix (200 MB at 128^3) streams past L1 and evict-first through L2, so that the vectors (67 MB)
-// stay there, and no part of L2 is set aside for it: with the persisting set-aside that the
-// global-memory form asks for, 128^3 takes 75 us per iteration instead of 52, and letting L2 keep
-// 15, 30, 50 or 100% of the slots gives 55, 61, 63, 64 (100^3, which nearly fits: 29.1 at 0%, 28.0 at
-// 30%).  us per iteration, global-memory form -> here: 128^3 FP32 99.7 -> 52.1, BF16 106 -> 54.8; 100^3
-// FP32 47.2 -> 29.1, BF16 42.4 -> 30.4; 1400^2 FP32 71.2 -> 33.9.  Of the 52: window 10, product 26
-// (DRAM: 200 MB at 6.5 TB/s is 31, part of it overlapping the window), barriers and totals 7, phase B 7.
+// The matrix (200 MB at 128^3) streams past L1 and through L2 at its default priority, beside the
+// vectors (67 MB), and no part of L2 is set aside for it: with the persisting set-aside that the
+// global-memory form asks for, 128^3 takes 73.5 us per iteration instead of 50.4 (104^3 reads 114 MB
+// of DRAM per iteration, its 107 MB of slots and little else).  us per iteration, global-memory form
+// -> here: 128^3 FP32 99.7 -> 52.1, BF16 106 -> 54.8; 100^3 FP32 47.2 -> 29.1, BF16 42.4 -> 30.4;
+// 1400^2 FP32 71.2 -> 33.9.  Of the 52: window 10, product 26 (DRAM: 200 MB at 6.5 TB/s is 31, part
+// of it overlapping the window), barriers and totals 7, phase B 7.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
