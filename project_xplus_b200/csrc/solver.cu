@@ -690,6 +690,8 @@ void ensure_trace(xplus_pcg* h, int cap) {
 void enqueue_solve(xplus_pcg* h, double tau, int tau_mode, int max_iters_in, int trace_rows, cudaStream_t st) {
     require(tau > 0.0 && tau == tau, XPLUS_ERR_ARG, "tau must be positive");
     require(tau_mode == XPLUS_TAU_ABS_RR || tau_mode == XPLUS_TAU_REL_TRUE, XPLUS_ERR_ARG, "bad tau_mode");
+    // the solve kernels' slice tables hold a slice's first slot in 32 bits (the product counts in 64)
+    require(h->slots < (1LL << 31), XPLUS_ERR_ARG, "matrix too large for a solve (2^31 slots)");
     const int max_iters = max_iters_in > 0 ? max_iters_in : std::max(4 * h->n, 1000);
     PcgArgs a{};
     a.n = h->n;
