@@ -99,9 +99,12 @@ typedef struct xplus_opts {
                               the last such handle restores the previous limit.  The limit is the
                               device's: a windowed solve beside such a handle is slower (128^3:
                               50 us per iteration alone, 74 beside one) */
-    int resident;          /* FP32 vectors, row-sum form: use the SM-resident kernel (state and
-                              the search direction's band + halo in shared memory) when one CTA
-                              per SM holds it (default 1) */
+    int resident;          /* FP32 vectors, row-sum form: use the kernels that keep in shared
+                              memory what fits there (default 1): the SM-resident one (state and
+                              the search direction's band + halo, when one CTA per SM holds it),
+                              beyond it the windowed one (band + halo of the search direction),
+                              and with G^T G the SM-resident form of that.  0: the global-memory
+                              kernels */
     int restart_on_replace; /* search direction after an FP64 residual replacement: 0 keeps it,
                               1 restarts it (p = z) after every replacement, 2 restarts it only
                               after replacements triggered by a replace_drop fall of ||r|| or by
@@ -189,7 +192,8 @@ int xplus_pcg_destroy(xplus_pcg* h);
 /* Blocking solve with host arrays.  x0 may be NULL (zeros).  max_iters <= 0 means
  * max(4n, 1000) as src/CgSolverGolden.hpp:47.  resid_hist (nullable, length hist_len)
  * receives sqrt(rr) after each iteration, the per-iteration residual of the golden
- * trace (src/CgSolverGolden.hpp:101-108).  metrics may be NULL. */
+ * trace (src/CgSolverGolden.hpp:101-108).  metrics may be NULL.  A solve, of whatever entry
+ * point, takes fewer than 2^31 stored slots (XPLUS_ERR_ARG; create and spmv take more). */
 int xplus_pcg_solve(xplus_pcg* h, const double* b, const double* x0, double tau, int tau_mode,
                     int max_iters, double* x_out, int* iters_out, double* resid_hist,
                     int hist_len, xplus_metrics* metrics);

@@ -14,8 +14,8 @@
 //   D   z = G^T t (halo t read), r'.z, publish z                                   -> grid barrier
 // In the global-memory form each phase was two dependent L2 round trips (slots, then records of the
 // own band too: the barrier's acquire empties L1).  us per iteration there -> here, FP32 values:
-// 300^2 16.8 -> 12.0, 600^2 27.2 -> 17.4, 900^2 51.9 -> 33.8 (less and less of the matrix fits); 4.4 of
-// the 12.0 us are the three grid barriers.
+// 300^2 16.7 -> 11.7, 600^2 26.1 -> 17.3, 900^2 50.9 -> 32.9 (less and less of the matrix fits); 4.3 of
+// the 11.7 us are the three grid barriers.
 // Shared memory per CTA: 20 bytes a row of the band, 12 a row of the window, then matrix slots.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

@@ -15,9 +15,9 @@
 // vectors (67 MB), and no part of L2 is set aside for it: with the persisting set-aside that the
 // global-memory form asks for, 128^3 takes 73.5 us per iteration instead of 50.4 (104^3 reads 114 MB
 // of DRAM per iteration, its 107 MB of slots and little else).  us per iteration, global-memory form
-// -> here: 128^3 FP32 99.7 -> 52.1, BF16 106 -> 54.8; 100^3 FP32 47.2 -> 29.1, BF16 42.4 -> 30.4;
-// 1400^2 FP32 71.2 -> 33.9.  Of the 52: window 10, product 26 (DRAM: 200 MB at 6.5 TB/s is 31, part
-// of it overlapping the window), barriers and totals 7, phase B 7.
+// -> here: 128^3 FP32 95.7 -> 50.0, BF16 100.6 -> 51.8; 100^3 FP32 46.4 -> 27.8, BF16 40.7 -> 29.0;
+// 1400^2 FP32 69.4 -> 32.7.  Of the 50 (median CTA): window and product 36 (DRAM: 200 MB at 6.5 TB/s
+// is 31), barriers and totals 6.6, phase B 6.8.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
